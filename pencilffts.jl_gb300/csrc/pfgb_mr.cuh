@@ -43,10 +43,10 @@ __host__ __device__ constexpr size_t mr_smem(int r0, int logn, int op) {
   return (size_t)r0 * mr_tw<R>(logn) * fast_pitch<R>(logn, op) * sizeof(Cx<R>);
 }
 
-// y_k = sum_j v_j exp(SIGN 2 pi i j k / R0) for odd R0, from the table of
-// exp(-2 pi i m / M), M = R0 N (the R0-th roots at multiples of N)
+// y_k = sum_j v_j exp(SIGN 2 pi i j k / R0) for odd R0, from the R0-th roots
+// exp(-2 pi i m / R0) (the first R0 entries of tw2)
 template <int R0, int SIGN, typename R>
-__device__ __forceinline__ void mr_dft_odd(Cx<R> (&v)[R0], const void* tw2, int N) {
+__device__ __forceinline__ void mr_dft_odd(Cx<R> (&v)[R0], const void* tw2) {
   constexpr int H = (R0 - 1) / 2;
   Cx<R> s[H], d[H];
   Cx<R> y0 = v[0];
@@ -63,7 +63,7 @@ __device__ __forceinline__ void mr_dft_odd(Cx<R> (&v)[R0], const void* tw2, int 
     Cx<R> a = v[0], b = mk(R(0), R(0));
 #pragma unroll
     for (int j = 1; j <= H; ++j) {
-      const Cx<R> w = ldg_tw<R>(tw2, ((j * k) % R0) * N);  // (cos t, -sin t)
+      const Cx<R> w = ldg_tw<R>(tw2, (j * k) % R0);  // (cos t, -sin t)
       a = a + mk(s[j - 1].re * w.re, s[j - 1].im * w.re);
       b = b - mk(d[j - 1].re * w.im, d[j - 1].im * w.im);  // sum d_j sin t
     }
@@ -141,56 +141,72 @@ __device__ __forceinline__ void mr_tile(const FastArgs& a, int64_t bid, Cx<R>* z
   }
 
   // ---- phase A: R0-point DFTs, twiddles, park in the sub-lines (a loop:
-  // nothing is held in registers across r) ----
+  // nothing is held in registers across its rounds).  The loads of a round's
+  // BA positions are issued before its stores to shared memory, which the
+  // compiler does not move them over: with one position a round the Float32
+  // 384-point passes waited for memory 8 times a tile (3 x 384^3 gradient
+  // 2.69 -> 2.59 ms) ----
+  constexpr int BA = IO::kDD ? 1 : OP == OP_C2R ? 2 : 4;
 #pragma unroll 1
-  for (int r = 0; r < 8; ++r) {
-    const int n1 = b + r * T;
-    Cx<R> u[R0];
+  for (int r0 = 0; r0 < 8; r0 += BA) {
+    MC ra[BA][R0], rb[BA][R0];
+    if (OP != OP_C2C || a.nterm == 0) {
 #pragma unroll
-    for (int n2 = 0; n2 < R0; ++n2) {
-      const int n = n1 + N * n2;
-      if constexpr (OP == OP_C2C) {
-        if (a.nterm > 0) {  // sum of i k_t src_t (fused divergence / curl)
-          u[n2] = mk(R(0), R(0));
-          for (int t = 0; t < a.nterm; ++t) {
-            const MC q = p < nvalid ? reinterpret_cast<const MC*>(a.tsrc[t])[ioff + (int64_t)n * ssa + (int64_t)p * sst]
-                                    : MC{0, 0};
-            const int64_t idx = a.trole[t] == 0   ? (int64_t)n
-                                : a.trole[t] == 1 ? t0 + p
-                                                  : outer_index(a, (unsigned)bid, a.trole[t] - 2);
-            u[n2] = u[n2] + mul_ik(mk(mkr<R>(q.x, emax), mkr<R>(q.y, emax)), idx, a.thalf[t], a.tn[t],
-                                   a.tk0_h[t], a.tk0_l[t]);
+      for (int q = 0; q < BA; ++q)
+#pragma unroll
+        for (int n2 = 0; n2 < R0; ++n2) {
+          const int n = b + (r0 + q) * T + N * n2;
+          ra[q][n2] = rb[q][n2] = MC{0, 0};
+          if constexpr (OP == OP_C2C) {
+            if (p < nvalid) ra[q][n2] = reinterpret_cast<const MC*>(a.in)[ioff + n * ssa + p * sst];
+          } else if constexpr (OP == OP_R2C) {
+            const MR* in = reinterpret_cast<const MR*>(a.in) + ioff + n * ssa;
+            if (2 * p < nvalid) ra[q][n2].x = in[(2 * p) * sst];
+            if (2 * p + 1 < nvalid) ra[q][n2].y = in[(2 * p + 1) * sst];
+          } else {  // C2R: Hermitian extension of two half spectra (m = M/2 + 1 inputs)
+            const MC* in = reinterpret_cast<const MC*>(a.in) + ioff + (n <= M / 2 ? n : M - n) * ssa;
+            if (2 * p < nvalid) ra[q][n2] = in[(2 * p) * sst];
+            if (2 * p + 1 < nvalid) rb[q][n2] = in[(2 * p + 1) * sst];
           }
-        } else {
-          const MC q = p < nvalid ? reinterpret_cast<const MC*>(a.in)[ioff + (int64_t)n * ssa + (int64_t)p * sst] : MC{0, 0};
-          u[n2] = mk(mkr<R>(q.x, emax), mkr<R>(q.y, emax));
         }
-        if (a.deriv == 1) {
-          const int64_t idx = a.deriv_role == 0 ? (int64_t)n : a.deriv_role == 1 ? t0 + p : didx;
-          u[n2] = mul_ik(u[n2], idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
-        }
-      } else if constexpr (OP == OP_R2C) {
-        const MR* in = reinterpret_cast<const MR*>(a.in) + ioff + (int64_t)n * ssa;
-        const MR qa = 2 * p < nvalid ? in[(int64_t)(2 * p) * sst] : MR(0);
-        const MR qb = 2 * p + 1 < nvalid ? in[(int64_t)(2 * p + 1) * sst] : MR(0);
-        u[n2] = mk(mkr<R>(qa, emax), mkr<R>(qb, emax));
-      } else {  // C2R: Hermitian extension of two half spectra (m = M/2 + 1 inputs)
-        const int k = n <= M / 2 ? n : M - n;
-        const MC* in = reinterpret_cast<const MC*>(a.in) + ioff + (int64_t)k * ssa;
-        const MC qa = 2 * p < nvalid ? in[(int64_t)(2 * p) * sst] : MC{0, 0};
-        const MC qb = 2 * p + 1 < nvalid ? in[(int64_t)(2 * p + 1) * sst] : MC{0, 0};
-        Cx<R> A = mk(mkr<R>(qa.x, emax), mkr<R>(qa.y, emax));
-        Cx<R> B = mk(mkr<R>(qb.x, emax), mkr<R>(qb.y, emax));
-        if (k == 0 || 2 * k == M) { A.im = R(0); B.im = R(0); }
-        if (n > M / 2) { A.im = -A.im; B.im = -B.im; }
-        u[n2] = mk(A.re - B.im, A.im + B.re);
-      }
     }
-    mr_dft_odd<R0, SIGN>(u, a.tw2, N);
 #pragma unroll
-    for (int k2 = 0; k2 < R0; ++k2) {
-      const Cx<R> y = k2 == 0 ? u[0] : tw_mul<R, SIGN>(u[k2], a.tw2, n1 * k2);
-      sub(k2)[sidx<R, LOGN, OP>(p, n1)] = y;
+    for (int q = 0; q < BA; ++q) {
+      const int n1 = b + (r0 + q) * T;
+      Cx<R> u[R0];
+#pragma unroll
+      for (int n2 = 0; n2 < R0; ++n2) {
+        const int n = n1 + N * n2;
+        u[n2] = mk(mkr<R>(ra[q][n2].x, emax), mkr<R>(ra[q][n2].y, emax));
+        if constexpr (OP == OP_C2C) {
+          if (a.nterm > 0) {  // sum of i k_t src_t (fused divergence / curl)
+            u[n2] = mk(R(0), R(0));
+            for (int t = 0; t < a.nterm; ++t) {
+              const MC x = p < nvalid ? reinterpret_cast<const MC*>(a.tsrc[t])[ioff + n * ssa + p * sst] : MC{0, 0};
+              const int64_t idx = a.trole[t] == 0   ? (int64_t)n
+                                  : a.trole[t] == 1 ? t0 + p
+                                                    : outer_index(a, (unsigned)bid, a.trole[t] - 2);
+              u[n2] = u[n2] + mul_ik(mk(mkr<R>(x.x, emax), mkr<R>(x.y, emax)), idx, a.thalf[t], a.tn[t],
+                                     a.tk0_h[t], a.tk0_l[t]);
+            }
+          }
+          if (a.deriv == 1) {
+            const int64_t idx = a.deriv_role == 0 ? (int64_t)n : a.deriv_role == 1 ? t0 + p : didx;
+            u[n2] = mul_ik(u[n2], idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
+          }
+        } else if constexpr (OP == OP_C2R) {
+          Cx<R> B = mk(mkr<R>(rb[q][n2].x, emax), mkr<R>(rb[q][n2].y, emax));
+          if (n == 0 || 2 * n == M) { u[n2].im = R(0); B.im = R(0); }
+          if (n > M / 2) { u[n2].im = -u[n2].im; B.im = -B.im; }
+          u[n2] = mk(u[n2].re - B.im, u[n2].im + B.re);
+        }
+      }
+      mr_dft_odd<R0, SIGN>(u, a.tw2);
+#pragma unroll
+      for (int k2 = 0; k2 < R0; ++k2) {
+        const Cx<R> y = k2 == 0 ? u[0] : tw_mul<R, SIGN>(u[k2], a.tw2, R0 + (k2 - 1) * N + n1);
+        sub(k2)[sidx<R, LOGN, OP>(p, n1)] = y;
+      }
     }
   }
 

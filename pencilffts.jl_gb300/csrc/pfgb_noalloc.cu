@@ -12,9 +12,9 @@
 // arrays, and the only other device memory the kernels touch is the
 // file-scope array below.
 //
-// Scratch: g_noalloc_scratch holds an exponent word and the double-float
-// twiddle tables of every power-of-two length 32..4096 (8160 entries of 16
-// bytes).  It is 130,816 bytes, resident on every GPU that loads the library
+// Scratch: g_noalloc_scratch holds an exponent word and the twiddle tables of
+// the register stages of every power-of-two length 32..4096 (8160 entries of
+// 16 bytes).  It is 130,816 bytes, resident on every GPU that loads the library
 // until the process exits.  Each line is scaled by its own largest exponent
 // (the kernel's per-line scaling), so lines of very different magnitude in
 // one batch keep their full accuracy; the exponent word only collects the
@@ -80,20 +80,20 @@ int setup_device(int dev, float** base) {
   void* ptr = nullptr;
   cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
   if (e != cudaSuccess) return fail_cuda(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
-  // double-float twiddles exp(-2 pi i m / M) for every supported M
+  // twiddles of the register stages for every supported M
   std::vector<float> tab(4 * (size_t)kTableEntries);
   const long double pi = 3.141592653589793238462643383279502884L;
   for (int lg = kNoAllocMinLog; lg <= kNoAllocMaxLog; ++lg) {
     const int M = 1 << lg;
     float* t = tab.data() + 4 * (size_t)(M - 32);
-    for (int m = 0; m < M; ++m) {
+    stage_twiddles(lg, 3, [&](int m) {  // M - 8 entries
       const long double a = 2.0L * pi * (long double)m / (long double)M;
       const long double c = cosl(a), s = -sinl(a);
-      t[4 * m + 0] = (float)c;
-      t[4 * m + 1] = (float)(c - (long double)(float)c);
-      t[4 * m + 2] = (float)s;
-      t[4 * m + 3] = (float)(s - (long double)(float)s);
-    }
+      *t++ = (float)c;
+      *t++ = (float)(c - (long double)(float)c);
+      *t++ = (float)s;
+      *t++ = (float)(s - (long double)(float)s);
+    });
   }
   e = cudaMemcpyToSymbol(g_noalloc_scratch, tab.data(), tab.size() * sizeof(float),
                          kHeaderFloats * sizeof(float), cudaMemcpyHostToDevice);

@@ -123,7 +123,7 @@ struct Pass {
   // mixed-radix register pass (mr_pass) for lines of r0 * 2^logn points
   bool mr = false;
   int r0 = 0, logn = 0;
-  const void* ftw2 = nullptr;  // its r0 * 2^logn-point twiddle table
+  const void* ftw2 = nullptr;  // its other twiddles (upload_mr_table); tensor-core form: the M-point table
   // Bluestein register pass (bs_pass) for other lines up to 2048 points:
   // convolution length 2^logl (ftw holds its twiddles), chirp and filter
   // tables; the generic kernel's geometry is kept (g_*) for executions it
@@ -382,6 +382,43 @@ static int upload_fast_table(pfgb_plan* P, int M, const void** out) {
   return PFGB_OK;
 }
 
+// The register stages' twiddles of a line of 2^logm points with 2^lp points a
+// thread (stage_twiddles), in the same format.
+static int upload_stage_table(pfgb_plan* P, int logm, int lp, const void** out) {
+  if (P->query_only) {
+    *out = nullptr;
+    return PFGB_OK;
+  }
+  const std::string key = (P->rb == 8 ? "stwdd" : "stwf") + std::to_string(logm) + "/" + std::to_string(lp);
+  auto it = P->tables.find(key);
+  if (it != P->tables.end()) {
+    *out = it->second;
+    return PFGB_OK;
+  }
+  std::vector<float> h;
+  h.reserve((size_t)4 << logm);
+  stage_twiddles(logm, lp, [&](int m) {
+    const std::complex<ld> w = expi_pi(2 * (int64_t)m, (int64_t)1 << logm);
+    for (ld c : {w.real(), w.imag()}) {
+      const float hi = (float)c;
+      h.push_back(hi);
+      if (P->rb == 8) h.push_back((float)(c - (ld)hi));
+    }
+  });
+  void* d = nullptr;
+  PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(float), 16)));
+  PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+  P->tables[key] = d;
+  *out = d;
+  return PFGB_OK;
+}
+// of a power-of-two pass (its points a thread) and of the other register
+// passes (8 points a thread)
+static int upload_fast_stages(pfgb_plan* P, int logm, const void** out) {
+  const int pts = P->rb == 8 ? fast_pts<dd>(logm) : fast_pts<float>(logm);
+  return upload_stage_table(P, logm, pts == 16 ? 4 : 3, out);
+}
+
 // A complex table in the register kernels' format (float (re, im), or dd
 // (re.hi, re.lo, im.hi, im.lo) for Float64 plans).
 static int upload_fast_vec(pfgb_plan* P, const std::string& key, const std::vector<std::complex<ld>>& v,
@@ -416,6 +453,20 @@ static int upload_fast_vec(pfgb_plan* P, const std::string& key, const std::vect
   P->tables[k] = d;
   *out = d;
   return PFGB_OK;
+}
+
+// Twiddles of the mixed-radix pass beside its sub-lines' stages, M = r0 n: the
+// r0-th roots exp(-2 pi i k / r0), then exp(-2 pi i k n1 / M) as entry
+// r0 + (k - 1) n + n1, k = 1 .. r0 - 1 (consecutive lanes: consecutive n1).
+static int upload_mr_table(pfgb_plan* P, int r0, int n, const void** out) {
+  const std::string key = "mr" + std::to_string(r0) + "/" + std::to_string(n);
+  std::vector<std::complex<ld>> t;
+  if (!P->query_only && !P->tables.count((P->rb == 8 ? "fvdd" : "fvf") + key)) {
+    for (int k = 0; k < r0; ++k) t.push_back(expi_pi(2 * k, r0));
+    for (int k = 1; k < r0; ++k)
+      for (int n1 = 0; n1 < n; ++n1) t.push_back(expi_pi(2 * (int64_t)k * n1, (int64_t)r0 * n));
+  }
+  return upload_fast_vec(P, key, t, out);
 }
 
 // Bluestein tables of a length-M DFT of sign `sign` with convolution length
@@ -481,25 +532,25 @@ static void bluestein_tables(int M, int L, int sign, std::vector<std::complex<ld
   for (auto& x : bf) x /= (ld)L;
 }
 
-// Twiddles of the fast kernel in fx form: exp(sign 2 pi i m / M) as
+// Twiddles of the register stages in fx form: exp(sign 2 pi i m / M) as
 // W = round(w 2^60) (clamped below 2^60) per part, stored as
 // (4 * (W >> 31), W & (2^31 - 1)) for the real and imaginary parts.
-static int upload_fast_table_fx(pfgb_plan* P, int M, int sign, const void** out) {
+static int upload_fast_table_fx(pfgb_plan* P, int logm, int sign, const void** out) {
   if (P->query_only) {
     *out = nullptr;
     return PFGB_OK;
   }
-  const std::string key = "ftwfx" + std::to_string(sign) + "_" + std::to_string(M);
+  const std::string key = "ftwfx" + std::to_string(sign) + "_" + std::to_string(logm);
   auto it = P->tables.find(key);
   if (it != P->tables.end()) {
     *out = it->second;
     return PFGB_OK;
   }
   std::vector<int32_t> h;
-  h.reserve((size_t)M * 4);
+  h.reserve((size_t)4 << logm);
   const ld two60 = std::ldexp((ld)1, 60);
-  for (int m = 0; m < M; ++m) {
-    const std::complex<ld> w = expi_pi(2 * (int64_t)m * (sign < 0 ? 1 : -1), M);
+  stage_twiddles(logm, 3, [&](int m) {
+    const std::complex<ld> w = expi_pi(2 * (int64_t)m * (sign < 0 ? 1 : -1), (int64_t)1 << logm);
     for (ld c : {w.real(), w.imag()}) {
       long long W = (long long)std::llround(c * two60);
       if (W > (1ll << 60) - 1) W = (1ll << 60) - 1;
@@ -507,9 +558,9 @@ static int upload_fast_table_fx(pfgb_plan* P, int M, int sign, const void** out)
       h.push_back((int32_t)(4 * (W >> 31)));
       h.push_back((int32_t)(W & 0x7FFFFFFFll));
     }
-  }
+  });
   void* d = nullptr;
-  PFGB_CUDA(cudaMalloc(&d, h.size() * sizeof(int32_t)));
+  PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(int32_t), 16)));
   PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
   P->tables[key] = d;
   *out = d;
@@ -658,7 +709,7 @@ static int bluestein_form(pfgb_plan* P, Pass& ps) {
   std::vector<std::complex<ld>> w, bf;
   bluestein_tables(M, 1 << logl, ps.sign, w, bf);
   const std::string key = std::to_string(M) + "/" + std::to_string(1 << logl) + (ps.sign > 0 ? "+" : "-");
-  int rc = upload_fast_table(P, 1 << logl, &ps.ftw);
+  int rc = upload_stage_table(P, logl, 3, &ps.ftw);
   if (!rc) rc = upload_fast_vec(P, "bsw" + key, w, &ps.bs_chirp);
   if (!rc) rc = upload_fast_vec(P, "bsf" + key, bf, &ps.bs_filt);
   if (rc) return rc;
@@ -766,7 +817,7 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
         w[j] = expi_pi(j, 2 * (int64_t)n);                   // c_j = exp(-i pi j / (2n))
         w[n + j] = expi_pi(2 * (int64_t)j + 1, 4 * (int64_t)n);  // d_j = exp(-i pi (2j+1) / (4n))
       }
-      int rc2 = upload_fast_table(P, 2 * n, &ps.ftw);
+      int rc2 = upload_fast_stages(P, ps.logm, &ps.ftw);
       if (!rc2) rc2 = upload_fast_vec(P, "d4/" + std::to_string(n), w, &ps.d23_tab);
       if (rc2) return rc2;
       const bool packed = fast_packed(ps.fop);
@@ -789,7 +840,7 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
       std::vector<std::complex<ld>> w(n);
       for (int k = 0; k < n; ++k)  // exp(-i pi k / (2n)); DHT: (1 + i) / 2
         w[k] = dht ? std::complex<ld>(0.5L, 0.5L) : expi_pi(k, 2 * (int64_t)n);
-      int rc2 = upload_fast_table(P, n, &ps.ftw);
+      int rc2 = upload_fast_stages(P, ps.logm, &ps.ftw);
       if (!rc2) rc2 = upload_fast_vec(P, (dht ? "dht/" : "d23/") + std::to_string(n), w, &ps.d23_tab);
       if (rc2) return rc2;
       const bool packed = fast_packed(ps.fop);
@@ -811,8 +862,8 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
     }
     ps.logm = 0;
     while ((1 << ps.logm) < M) ++ps.logm;
-    rc = upload_fast_table(P, M, &ps.ftw);
-    if (!rc && P->fx) rc = upload_fast_table_fx(P, M, ps.sign, &ps.ftw_fx);
+    rc = upload_fast_stages(P, ps.logm, &ps.ftw);
+    if (!rc && P->fx) rc = upload_fast_table_fx(P, ps.logm, ps.sign, &ps.ftw_fx);
     if (rc) return rc;
     const bool packed = fast_packed(ps.fop);
     ps.clines = P->rb == 8 ? fast_tw<dd>(ps.logm, ps.fop) : fast_tw<float>(ps.logm, ps.fop);
@@ -823,6 +874,7 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
       ps.tc = true;
       ps.clines = ps.lines = tc_lines(ps.logm);
       rc = upload_tc_table(P, ps.logm, ps.sign, &ps.tcb);
+      if (!rc) rc = upload_fast_table(P, M, &ps.ftw2);
       if (rc) return rc;
     }
     return PFGB_OK;
@@ -841,8 +893,8 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
       ps.r0 = r0;
       ps.logn = 0;
       while ((1 << ps.logn) < n) ++ps.logn;
-      rc = upload_fast_table(P, n, &ps.ftw);
-      if (!rc) rc = upload_fast_table(P, M, &ps.ftw2);
+      rc = upload_stage_table(P, ps.logn, 3, &ps.ftw);
+      if (!rc) rc = upload_mr_table(P, r0, n, &ps.ftw2);
       if (rc) return rc;
       const bool packed = fast_packed(ps.op);
       ps.clines = P->rb == 8 ? mr_tw<dd>(ps.logn) : mr_tw<float>(ps.logn);

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256, 2) tc_pass(const FastArgs a) {
     const float4* src = reinterpret_cast<const float4*>(a.tcb);
     float4* dst = reinterpret_cast<float4*>(Bs);
     for (int i = tid; i < C::BBYTES / 16; i += 256) dst[i] = src[i];
-    const float2* tw = reinterpret_cast<const float2*>(a.tw);
+    const float2* tw = reinterpret_cast<const float2*>(a.tw2);
     for (int i = tid; i < M; i += 256) {
       float2 w = tw[i];
       if (SIGN > 0) w.y = -w.y;

@@ -335,7 +335,7 @@ int pfgb_plan_get_timing(pfgb_plan* plan, pfgb_pass_timing* out, int max, int* n
  * `n` complex doubles (interleaved re, im) from `in` to `out` (in == out
  * allowed), sign -1 (FFT) or +1 (BFFT, unnormalised), on `stream`, computing
  * in double-float like the Float64 plans.  Its only scratch is a fixed
- * 130,816-byte static device array (exponent word + twiddle tables), so n
+ * 391,936-byte static device array (exponent word + twiddle tables), so n
  * must be a power of two in [32, 4096]; other sizes return PFGB_ERR_ARGUMENT.
  * Each line is scaled by its own largest exponent, so lines of very
  * different magnitude in one batch keep their accuracy.  The first call on a

@@ -24,6 +24,7 @@
 #include "pfgb_dd.cuh"
 #include "pfgb_device.cuh"
 #include "pfgb_fx.cuh"
+#include "pfgb_xf.cuh"
 
 namespace pfgb {
 
@@ -57,6 +58,10 @@ struct FastArgs {
   int vec2;          // float r2c: lines 2j, 2j+1 adjacent and 16-byte aligned in the output
   int scale_on;
   float scale_h, scale_l;  // ldiv! normalisation as hi + lo
+  // double outputs of an xf pass: its significand for xf_scaled, and the
+  // exponent that goes with it
+  int scale_xw, scale_xe;
+  float scale_xo, scale_xf;
   // Float64 (dd) passes: the input / output of a pass between two dd passes is
   // kept in dd form (re.hi, re.lo, im.hi, im.lo floats), scaled by the power
   // of two 2^(1023 - *emax), *emax the run exponent (see self_scale below).
@@ -297,6 +302,10 @@ __device__ __forceinline__ Cx<R> tw_mul(Cx<R> v, const void* tw, int m) {
     const int4 q = __ldg(reinterpret_cast<const int4*>(tw) + m);
     fx_twiddle(v.re, v.im, fx_tw{q.x, q.y, q.z, q.w});
     return v;
+  } else if constexpr (std::is_same<R, xf>::value) {  // the product in units 2^s times larger
+    const int4 q = __ldg(reinterpret_cast<const int4*>(tw) + m);
+    xf_twiddle<(SIGN > 0)>(v.re, v.im, xf_tw{q.x, q.y, __int_as_float(q.z), __int_as_float(q.w)});
+    return v;
   } else {
     Cx<R> w = ldg_tw<R>(tw, m);
     if (SIGN > 0) w = conj(w);
@@ -347,6 +356,66 @@ __device__ __forceinline__ void line_sync(bool lanes_across_lines, int p) {
   }
 }
 
+// Largest m of the threads of a double-float line, in two steps around a
+// barrier of the line (line_sync): put leaves this thread's or warp's part in
+// red (the parts of line p at p N .. p N + N - 1, read back in vectors), get
+// collects the line's.  red: one word a thread, 16-byte aligned.
+template <int LOGM, int OP, bool ACROSS>
+__host__ __device__ constexpr int line_parts() {
+  constexpr int T = (1 << LOGM) / 8;
+  return ACROSS ? (fast_tw<dd>(LOGM, OP) >= 32 ? T : fast_threads<dd>(LOGM, OP) / 32) : (T > 32 ? T / 32 : 1);
+}
+template <int N>
+__device__ __forceinline__ unsigned max_of(unsigned m, const unsigned* q) {
+  if constexpr (N >= 4) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+      const uint4 v = *reinterpret_cast<const uint4*>(q + i);
+      m = __vimax3_u32(__vimax3_u32(m, v.x, v.y), v.z, v.w);
+    }
+  } else if constexpr (N == 2) {
+    const uint2 v = *reinterpret_cast<const uint2*>(q);
+    m = __vimax3_u32(m, v.x, v.y);
+  }
+  return m;
+}
+template <int LOGM, int OP>
+__device__ __forceinline__ unsigned line_max_put(unsigned m, unsigned* red, bool lanes_across_lines, int p) {
+  constexpr int T = (1 << LOGM) / 8;
+  constexpr int TH = fast_threads<dd>(LOGM, OP);
+  constexpr int TW = fast_tw<dd>(LOGM, OP);
+  const int tid = threadIdx.x;
+  if (T == 1) return m;
+  if (lanes_across_lines && T != TH) {
+    constexpr int N = line_parts<LOGM, OP, true>();
+    if constexpr (TW >= 32) {
+      red[p * N + tid / TW] = m;
+    } else {
+#pragma unroll
+      for (int o = TW; o < 32; o *= 2) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+      if ((tid & 31) < TW) red[p * N + (tid >> 5)] = m;
+    }
+  } else if constexpr (T <= 32) {
+    const unsigned mask = T == 32 ? 0xFFFFFFFFu : ((1u << (T & 31)) - 1u) << ((p * T) & 31);
+    m = __reduce_max_sync(mask, m);
+  } else {
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    if ((tid & 31) == 0) red[tid >> 5] = m;
+  }
+  return m;
+}
+template <int LOGM, int OP>
+__device__ __forceinline__ unsigned line_max_get(unsigned m, const unsigned* red, bool lanes_across_lines, int p) {
+  constexpr int T = (1 << LOGM) / 8;
+  if (T == 1) return m;
+  if (lanes_across_lines && T != fast_threads<dd>(LOGM, OP)) {
+    constexpr int N = line_parts<LOGM, OP, true>();
+    return max_of<N>(m, red + p * N);
+  }
+  constexpr int N = line_parts<LOGM, OP, false>();
+  return N > 1 ? max_of<N>(m, red + p * N) : m;
+}
+
 // The register stages of a line of M = 2^LOGM points, P points a thread
 // (positions b + r M/P): radix-P stages (dft8 or dft16), then one radix-2,
 // 4 or 8 stage when log2 M is not a multiple of log2 P; outputs left in
@@ -359,10 +428,13 @@ __device__ __forceinline__ void line_sync(bool lanes_across_lines, int p) {
 // the 32 lanes of a load touch up to r times as many 128-byte lines, 28
 // against 7 per 16 lanes and radix-8 stage; the Float32 passes are bound by
 // these lookups and the exchanges (round trips: 512^3 Float32 1.41 -> 1.26 ms,
-// 1024^3 13.2 -> 11.0 ms, 512^3 Float64 4.40 -> 4.14 ms).
-template <typename R, int LOGM, int SIGN, int OP, int P = 8, bool ZH = false>
-__device__ __forceinline__ void fast_stages(Cx<R> (&v)[P], Cx<R>* z, int p, int b, const void* tw,
-                                            bool lanes_across_lines) {
+// 1024^3 13.2 -> 11.0 ms, 512^3 Float64 4.40 -> 4.14 ms).  R = xf: the line's
+// shifts (pfgb_xf.cuh) are added to shifts, HEAD more bits are kept free; red:
+// one word a thread.
+template <typename R, int LOGM, int SIGN, int OP, int P, bool ZH, int HEAD = 0>
+__device__ __forceinline__ void stages_core(Cx<R> (&v)[P], Cx<R>* z, int p, int b, const void* tw,
+                                            bool lanes_across_lines, unsigned* red, int& shifts) {
+  constexpr bool XF = std::is_same<R, xf>::value;
   static_assert(!ZH || P == 8, "zero upper half: 8 points a thread");
   constexpr int M = 1 << LOGM;
   constexpr int T = M / P;
@@ -371,15 +443,19 @@ __device__ __forceinline__ void fast_stages(Cx<R> (&v)[P], Cx<R>* z, int p, int 
   constexpr int REM = LOGM % LP;
   constexpr int NST = SP + (REM ? 1 : 0);
   int Ls = 1;
+  int sh = 0;         // xf: shift of the stage's twiddles
+  unsigned lmax = 0;  // xf: largest component of the line
 #pragma unroll
   for (int s = 0; s < NST; ++s) {
     const bool last = (s == NST - 1);
+    const void* tws = XF && s > 0 ? reinterpret_cast<const int4*>(tw) + (sh - 1) * (M - P) : tw;
     if (s < SP) {
       const int j = b & (Ls - 1);
       if (Ls > 1) {
         const int e0 = Ls - P + j;  // the stage's first entry (Ls - P), lane j
 #pragma unroll
-        for (int r = 1; r < P; ++r) v[r] = tw_mul<R, SIGN>(v[r], tw, e0 + (r - 1) * Ls);
+        for (int r = 1; r < P; ++r) v[r] = tw_mul<R, SIGN>(v[r], tws, e0 + (r - 1) * Ls);
+        if constexpr (XF) v[0] = mk(xf_shift(v[0].re, sh), xf_shift(v[0].im, sh));
       }
       if constexpr (P == 16) dft16<SIGN>(v);
       else if (ZH && s == 0) dft8_zh<SIGN>(v);
@@ -399,7 +475,8 @@ __device__ __forceinline__ void fast_stages(Cx<R> (&v)[P], Cx<R>* z, int p, int 
         const int beta = Ls - P + b + r1 * T;
 #pragma unroll
         for (int q = 1; q < RS; ++q)
-          v[r1 + q * G] = tw_mul<R, SIGN>(v[r1 + q * G], tw, beta + (q - 1) * (M / RS));
+          v[r1 + q * G] = tw_mul<R, SIGN>(v[r1 + q * G], tws, beta + (q - 1) * (M / RS));
+        if constexpr (XF) v[r1] = mk(xf_shift(v[r1].re, sh), xf_shift(v[r1].im, sh));
         if constexpr (RS == 2) {
           dft2<SIGN>(v[r1], v[r1 + G]);
         } else if constexpr (RS == 4) {
@@ -415,12 +492,63 @@ __device__ __forceinline__ void fast_stages(Cx<R> (&v)[P], Cx<R>* z, int p, int 
       }
     }
     if (!last) {
+      if constexpr (XF) {
+        int hi = 0, lo = 0;
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+          hi = __vimax3_s32(hi, v[r].re.h, v[r].im.h);
+          lo = __vimin3_s32(lo, v[r].re.h, v[r].im.h);
+        }
+        lmax = line_max_put<LOGM, OP>((unsigned)max(hi, ~lo), red, lanes_across_lines, p);
+      }
       line_sync<R, LOGM, OP, P>(lanes_across_lines, p);
       const int zr = sidx<R, LOGM, OP>(p, b);
 #pragma unroll
       for (int r = 0; r < P; ++r) v[r] = xld<R, LOGM, OP>(z, zr + padded<R, LOGM>(r * T));
+      if constexpr (XF) {
+        lmax = line_max_get<LOGM, OP>(lmax, red, lanes_across_lines, p);
+        sh = xf_stage_shift(lmax, (s + 1 < SP ? 3 : REM) + HEAD);
+        shifts += sh;
+      }
       line_sync<R, LOGM, OP, P>(lanes_across_lines, p);
     }
+  }
+}
+
+// A double-float line's values in xf, scaled by the line's largest high part;
+// returns its biased float exponent (at least 27, plus HEAD).
+template <int LOGM, int OP, int NIN, int HEAD = 0>
+__device__ __forceinline__ unsigned line_to_xf(const Cx<dd> (&v)[8], Cx<xf> (&x)[8], unsigned* red,
+                                               bool lanes_across_lines, int p) {
+  float mf = 0.0f;  // (a NaN is in the fractions: xf_line_exp)
+#pragma unroll
+  for (int r = 0; r < NIN; ++r) mf = fmaxf(fmaxf(mf, fabsf(v[r].re.h)), fabsf(v[r].im.h));
+  const unsigned m = line_max_put<LOGM, OP>(__float_as_uint(mf), red, lanes_across_lines, p);
+  if constexpr (LOGM > 3) line_sync<dd, LOGM, OP>(lanes_across_lines, p);
+  const unsigned e = xf_line_exp(line_max_get<LOGM, OP>(m, red, lanes_across_lines, p)) + HEAD;
+  const float f = xf_scale_in(e);
+#pragma unroll
+  for (int r = 0; r < NIN; ++r) x[r] = mk(dd2xf(v[r].re, f), dd2xf(v[r].im, f));
+  return e;
+}
+
+// The stages of a line: in xf for double-float lines (converted with the
+// line's own scale, and back to the scale the line came in), else in R.
+template <typename R, int LOGM, int SIGN, int OP, int P = 8, bool ZH = false>
+__device__ __forceinline__ void fast_stages(Cx<R> (&v)[P], Cx<R>* z, int p, int b, const void* tw,
+                                            bool lanes_across_lines) {
+  int shifts = 0;
+  if constexpr (std::is_same<R, dd>::value) {
+    __shared__ __align__(16) unsigned red[2][fast_threads<dd>(LOGM, OP)];
+    Cx<xf> x[P];
+    const unsigned e = line_to_xf<LOGM, OP, ZH ? P / 2 : P>(v, x, red[0], lanes_across_lines, p);
+    stages_core<xf, LOGM, SIGN, OP, P, ZH>(x, reinterpret_cast<Cx<xf>*>(z), p, b, tw, lanes_across_lines, red[1],
+                                           shifts);
+    const unsigned ue = xf_unit_exp(e) + (unsigned)shifts;
+#pragma unroll
+    for (int r = 0; r < P; ++r) v[r] = mk(xf2dd(x[r].re, ue), xf2dd(x[r].im, ue));
+  } else {
+    stages_core<R, LOGM, SIGN, OP, P, ZH>(v, z, p, b, tw, lanes_across_lines, nullptr, shifts);
   }
 }
 
@@ -688,8 +816,12 @@ __device__ __forceinline__ void fast_tile_load(const FastArgs& a, int64_t bid, c
       // exponents of the elements' first-pass lines, loaded ahead of the data
       int tev[P];
       if (IO::kDD && a.te_rescale) {
+        // (b + r T) >> sh = (b >> sh) + r (T >> sh): sh is 0, 1 (pairs of real
+        // lines), or the factor is 0
+        const unsigned te0 = te_index(a, o.tebase, t0 + p, b), dte = ((unsigned)T >> a.te_sh[0]) * a.te_mul[0];
 #pragma unroll
-        for (int r = 0; r < P; ++r) tev[r] = p < nvalid ? __ldg(a.te + te_index(a, o.tebase, t0 + p, b + r * T)) : emax;
+        for (int r = 0; r < P; ++r)
+          tev[r] = p < nvalid ? __ldg(a.te + (T > 1 ? te0 + r * dte : te_index(a, o.tebase, t0 + p, r))) : emax;
       }
 #pragma unroll
       for (int r = 0; r < P; ++r) {
@@ -1357,6 +1489,182 @@ __device__ __forceinline__ void fast_tile_store(const FastArgs& a, int64_t bid, 
   }
 }
 
+// Operations of a double-float pass whose tile stays in xf from the load to
+// the store (fast_tile_xf); the others convert around their stages.
+__host__ __device__ constexpr bool fast_xf_op(int op) { return op == OP_C2C || op == OP_R2C || op == OP_C2R; }
+
+// One tile of a dd pass of these operations: doubles are converted to xf with
+// their line's own exponent (recorded for the next pass), dd inputs with
+// their line's largest high part; the r2c split is done in xf, and the
+// outputs go to dd or double form from xf.  Against converting to dd around
+// the stages: 512^3 Float64 round trip 3.56 -> 3.45 ms, and the
+// errors of a pass 4 times smaller.
+template <int LOGM, int SIGN, int OP, int IOM>
+__device__ __forceinline__ void fast_tile_xf(const FastArgs& a, int64_t bid, Cx<dd>* z, const void* src,
+                                             int64_t soff, int64_t ssa, int64_t sst) {
+  constexpr bool IN_DD = (IOM & 1) != 0, OUT_DD = (IOM & 2) != 0;
+  constexpr int M = 1 << LOGM;
+  constexpr int T = M / 8;
+  constexpr int TW = fast_tw<dd>(LOGM, OP);
+  constexpr int TH = fast_threads<dd>(LOGM, OP);
+  // the r2c split adds two outputs of a line: one more bit kept free
+  constexpr int HEAD = OP == OP_R2C ? 1 : 0;
+  const int tid = threadIdx.x;
+  const bool lanes = a.lmap_tile != 0;
+  int p, b;
+  if (lanes) { p = tid % TW; b = tid / TW; } else { b = tid % T; p = tid / T; }
+  FastTile s = fast_tile_begin<dd, LOGM, OP>(a, bid, soff, true);
+  __shared__ __align__(16) unsigned red[2][TH];
+  __shared__ int lue[TW], loff[TW], lexp[TW];
+  Cx<xf> x[8];
+  int ue;  // biased float exponent of the unit in the scale of the dd form
+  if constexpr (!IN_DD && OP != OP_C2R) {
+    double2 raw[8];
+    if constexpr (OP == OP_C2C) {
+      const double2* in = reinterpret_cast<const double2*>(src) + s.ioff + (int64_t)p * sst;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) raw[r] = p < s.nvalid ? in[b * ssa + r * (T * ssa)] : double2{0, 0};
+    } else {
+      const double* in = reinterpret_cast<const double*>(src) + s.ioff;
+      const int i0 = 2 * p, i1 = 2 * p + 1;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int64_t off = b * ssa + r * (T * ssa);
+        raw[r].x = i0 < s.nvalid ? in[off + (int64_t)i0 * sst] : 0.0;
+        raw[r].y = i1 < s.nvalid ? in[off + (int64_t)i1 * sst] : 0.0;
+      }
+    }
+    unsigned m = 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) m = max(m, max(dexp_u(raw[r].x), dexp_u(raw[r].y)));
+    m = line_max_put<LOGM, OP>(m, red[0], lanes, p);
+    if constexpr (LOGM > 3) line_sync<dd, LOGM, OP>(lanes, p);
+    s.emax = (int)line_max_get<LOGM, OP>(m, red[0], lanes, p);
+    s.emax_out = s.emax + a.emax_shift;
+    if (b == 0 && p < s.ncl_valid) {  // the line's leader: its exponent for the next pass and the run
+      if (a.te) a.te[s.t0 / (fast_packed(OP) ? 2 : 1) + p + a.te_ncl * div31((unsigned)bid, a.div_tiles)] = s.emax;
+      if (s.emax > *reinterpret_cast<const volatile int*>(a.emax_ptr)) atomicMax(const_cast<int*>(a.emax_ptr), s.emax);
+    }
+    const float fs = xf_frac_scale(s.emax);
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+      x[r] = mk(d2xf<26 - HEAD>(raw[r].x, s.emax, fs), d2xf<26 - HEAD>(raw[r].y, s.emax, fs));
+    ue = 101 + HEAD;
+    if (OP == OP_C2C && a.deriv == 1) {
+      Cx<dd> v[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const int64_t idx = a.deriv_role == 0 ? (int64_t)(b + r * T) : a.deriv_role == 1 ? s.t0 + p : s.didx;
+        v[r] = mul_ik(mk(xf2dd(x[r].re, 101u), xf2dd(x[r].im, 101u)), idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
+      }
+      ue = (int)xf_unit_exp(line_to_xf<LOGM, OP, 8>(v, x, red[1], lanes, p));
+      line_sync<dd, LOGM, OP>(lanes, p);  // red[1] is used again below
+    }
+  } else {
+    Cx<dd> v[8];
+    fast_tile_load<dd, LOGM, SIGN, OP, IOM>(a, bid, src, ssa, sst, p, b, s, v);
+    ue = (int)xf_unit_exp(line_to_xf<LOGM, OP, 8, HEAD>(v, x, red[0], lanes, p));
+  }
+  int shifts = 0;
+  stages_core<xf, LOGM, SIGN, OP, 8, false, HEAD>(x, reinterpret_cast<Cx<xf>*>(z), p, b, a.tw, lanes, red[1], shifts);
+  ue += shifts;
+
+  // ---- store ----
+  if (OP == OP_C2C && a.deriv == 2) {
+    Cx<dd> v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = mk(xf2dd(x[r].re, (unsigned)ue), xf2dd(x[r].im, (unsigned)ue));
+    if (b == 0) lexp[p] = s.emax;
+    fast_tile_store<dd, LOGM, SIGN, OP, IOM>(a, bid, p, b, s, v, z, lexp);
+    return;
+  }
+  // doubles: the unit's exponent with the line's, and the normalisation
+  auto to_double = [&](Cx<xf> y, int off) {
+    if (a.scale_on) y = mk(xf_scaled(y.re, a.scale_xw, a.scale_xo, a.scale_xf), xf_scaled(y.im, a.scale_xw, a.scale_xo, a.scale_xf));
+    double2 o;
+    xf2d(y, off, o.x, o.y);
+    return o;
+  };
+  auto to_dd4 = [](Cx<xf> y, int u) { return st_dd4(mk(xf2dd(y.re, (unsigned)u), xf2dd(y.im, (unsigned)u))); };
+  const int off = ue + s.emax_out - 254 + a.scale_xe;
+  if (a.store_direct && OP != OP_R2C) {
+    if constexpr (OP == OP_C2C) {
+      if (p < s.nvalid) {
+        const int64_t o0 = s.ooff + (int64_t)p * a.out_st + b * a.out_sa;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          if constexpr (OUT_DD) reinterpret_cast<float4*>(a.out)[o0 + r * (T * a.out_sa)] = to_dd4(x[r], ue);
+          else reinterpret_cast<double2*>(a.out)[o0 + r * (T * a.out_sa)] = to_double(x[r], off);
+        }
+      }
+    } else {  // C2R, real outputs of lines 2p and 2p + 1
+      double* out = reinterpret_cast<double*>(a.out) + s.ooff;
+      const int i0 = 2 * p, i1 = 2 * p + 1;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const double2 y = to_double(x[r], off);
+        const int64_t o = b * a.out_sa + r * (T * a.out_sa);
+        if (i0 < s.nvalid) out[o + (int64_t)i0 * a.out_st] = y.x;
+        if (i1 < s.nvalid) out[o + (int64_t)i1 * a.out_st] = y.y;
+      }
+    }
+    return;
+  }
+  // via shared memory: transposed layouts and the r2c split
+  Cx<xf>* zx = reinterpret_cast<Cx<xf>*>(z);
+  {
+    Cx<xf>* zw = zx + sidx<xf, LOGM, OP>(p, b);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) zw[padded<xf, LOGM>(r * T)] = x[r];
+  }
+  if (b == 0) {
+    lue[p] = ue;
+    loff[p] = off;
+  }
+  __syncthreads();
+  if constexpr (OP == OP_C2C) {
+#pragma unroll 2
+    for (int e = tid; e < TW * M; e += TH) {
+      int i, k;
+      if (a.out_tfast) { i = e % TW; k = e / TW; } else { k = e % M; i = e / M; }
+      if (i >= s.nvalid) continue;
+      const Cx<xf> y = zx[sidx<xf, LOGM, OP>(i, k)];
+      const int64_t o = s.ooff + (int64_t)k * a.out_sa + (int64_t)i * a.out_st;
+      if constexpr (OUT_DD) reinterpret_cast<float4*>(a.out)[o] = to_dd4(y, lue[i]);
+      else reinterpret_cast<double2*>(a.out)[o] = to_double(y, loff[i]);
+    }
+  } else if constexpr (OP == OP_R2C) {
+    constexpr int m = M / 2 + 1;  // n_out of a power-of-two r2c line
+    for (int e = tid; e < TW * m; e += TH) {
+      int q, k;
+      if (a.out_tfast) { q = e % TW; k = e / TW; } else { k = e % m; q = e / m; }
+      const Cx<xf> f = zx[sidx<xf, LOGM, OP>(q, k)];
+      const Cx<xf> g = conj(zx[sidx<xf, LOGM, OP>(q, k == 0 ? 0 : M - k)]);
+      const Cx<xf> A = f + g, B = mul_mi(f - g);  // (the factor 1/2: emax_shift)
+      const int64_t o = s.ooff + (int64_t)k * a.out_sa + (int64_t)(2 * q) * a.out_st;
+      if constexpr (OUT_DD) {
+        const int u = lue[q];
+        if (2 * q < s.nvalid) reinterpret_cast<float4*>(a.out)[o] = to_dd4(A, u);
+        if (2 * q + 1 < s.nvalid) reinterpret_cast<float4*>(a.out)[o + a.out_st] = to_dd4(B, u);
+      } else {
+        const int u = loff[q];
+        if (2 * q < s.nvalid) reinterpret_cast<double2*>(a.out)[o] = to_double(A, u);
+        if (2 * q + 1 < s.nvalid) reinterpret_cast<double2*>(a.out)[o + a.out_st] = to_double(B, u);
+      }
+    }
+  } else {  // C2R with a transposed output layout
+    double* out = reinterpret_cast<double*>(a.out) + s.ooff;
+    for (int e = tid; e < TW * M; e += TH) {
+      int q, k;
+      if (a.out_tfast) { q = e % TW; k = e / TW; } else { k = e % M; q = e / M; }
+      const double2 y = to_double(zx[sidx<xf, LOGM, OP>(q, k)], loff[q]);
+      const int64_t o = (int64_t)k * a.out_sa + (int64_t)(2 * q) * a.out_st;
+      if (2 * q < s.nvalid) out[o] = y.x;
+      if (2 * q + 1 < s.nvalid) out[o + a.out_st] = y.y;
+    }
+  }
+}
+
 // One tile of the register pass for float and dd (fx: fast_tile_fx): load
 // (from `src`: the pass input in global memory, or a copy of the tile's input
 // lines in shared memory), stages, store.  `src` is addressed as
@@ -1679,6 +1987,7 @@ template <typename R, int LOGM, int SIGN, int OP, int IOM>
 __device__ __forceinline__ void fast_tile(const FastArgs& a, int64_t bid, Cx<R>* z, const void* src,
                                           int64_t soff, int64_t ssa, int64_t sst) {
   if constexpr (FastIO<R>::kFX) fast_tile_fx<LOGM, SIGN, OP, IOM>(a, bid, z, src, soff, ssa, sst);
+  else if constexpr (FastIO<R>::kDD && fast_xf_op(OP)) fast_tile_xf<LOGM, SIGN, OP, IOM>(a, bid, z, src, soff, ssa, sst);
   else fast_tile_std<R, LOGM, SIGN, OP, IOM>(a, bid, z, src, soff, ssa, sst);
 }
 

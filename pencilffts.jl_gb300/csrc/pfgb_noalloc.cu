@@ -13,8 +13,8 @@
 // file-scope array below.
 //
 // Scratch: g_noalloc_scratch holds an exponent word and the twiddle tables of
-// the register stages of every power-of-two length 32..4096 (8160 entries of
-// 16 bytes).  It is 130,816 bytes, resident on every GPU that loads the library
+// the register stages of every power-of-two length 32..4096 (24480 entries of
+// 16 bytes).  It is 391,936 bytes, resident on every GPU that loads the library
 // until the process exits.  Each line is scaled by its own largest exponent
 // (the kernel's per-line scaling), so lines of very different magnitude in
 // one batch keep their full accuracy; the exponent word only collects the
@@ -34,6 +34,7 @@
 // cached address and tables would belong to the released context.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <complex>
 #include <cstring>
@@ -54,13 +55,13 @@ namespace {
 
 constexpr int kNoAllocMinLog = 5;   // 32 points
 constexpr int kNoAllocMaxLog = 12;  // 4096 points
-constexpr int kTableEntries = (1 << (kNoAllocMaxLog + 1)) - (1 << kNoAllocMinLog);  // 8160
+constexpr int kTableEntries = kXfShifts * ((1 << (kNoAllocMaxLog + 1)) - (1 << kNoAllocMinLog));  // 24480
 constexpr int kHeaderFloats = 64;   // exponent word, padded to 256 bytes
 constexpr int kScratchFloats = kHeaderFloats + 4 * kTableEntries;
 constexpr int kMaxDevices = 64;
 
 // [0]: exponent word (int, written, never read for results); from float 64 on: tables, the one of length M at
-// entry offset M - 32, entries (re.hi, re.lo, im.hi, im.lo).
+// entry offset 3 (M - 32), entries xf_tw.
 static __device__ __align__(256) float g_noalloc_scratch[kScratchFloats];
 
 struct DeviceState {
@@ -85,15 +86,13 @@ int setup_device(int dev, float** base) {
   const long double pi = 3.141592653589793238462643383279502884L;
   for (int lg = kNoAllocMinLog; lg <= kNoAllocMaxLog; ++lg) {
     const int M = 1 << lg;
-    float* t = tab.data() + 4 * (size_t)(M - 32);
-    stage_twiddles(lg, 3, [&](int m) {  // M - 8 entries
-      const long double a = 2.0L * pi * (long double)m / (long double)M;
-      const long double c = cosl(a), s = -sinl(a);
-      *t++ = (float)c;
-      *t++ = (float)(c - (long double)(float)c);
-      *t++ = (float)s;
-      *t++ = (float)(s - (long double)(float)s);
-    });
+    std::vector<float> t;
+    for (int sh = 1; sh <= kXfShifts; ++sh)
+      stage_twiddles(lg, 3, [&](int m) {  // M - 8 entries
+        const long double a = 2.0L * pi * (long double)m / (long double)M;
+        push_xf_twiddle(t, std::complex<long double>(cosl(a), -sinl(a)), sh);
+      });
+    std::copy(t.begin(), t.end(), tab.begin() + 4 * (size_t)kXfShifts * (M - 32));
   }
   e = cudaMemcpyToSymbol(g_noalloc_scratch, tab.data(), tab.size() * sizeof(float),
                          kHeaderFloats * sizeof(float), cudaMemcpyHostToDevice);
@@ -132,7 +131,7 @@ extern "C" int pfgb_fft1d_noalloc(int sign, int64_t n, int64_t howmany, void* ou
   int rc = setup_device(dev, &base);
   if (rc) return rc;
   int* emax = reinterpret_cast<int*>(base);
-  const float* tw = base + kHeaderFloats + 4 * (size_t)(n - 32);
+  const float* tw = base + kHeaderFloats + 4 * (size_t)kXfShifts * (n - 32);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   FastArgs A;
   std::memset(&A, 0, sizeof(A));

@@ -383,7 +383,8 @@ static int upload_fast_table(pfgb_plan* P, int M, const void** out) {
 }
 
 // The register stages' twiddles of a line of 2^logm points with 2^lp points a
-// thread (stage_twiddles), in the same format.
+// thread (stage_twiddles): float (re, im), or xf_tw for Float64 plans, one table
+// per shift.
 static int upload_stage_table(pfgb_plan* P, int logm, int lp, const void** out) {
   if (P->query_only) {
     *out = nullptr;
@@ -396,15 +397,18 @@ static int upload_stage_table(pfgb_plan* P, int logm, int lp, const void** out) 
     return PFGB_OK;
   }
   std::vector<float> h;
-  h.reserve((size_t)4 << logm);
-  stage_twiddles(logm, lp, [&](int m) {
-    const std::complex<ld> w = expi_pi(2 * (int64_t)m, (int64_t)1 << logm);
-    for (ld c : {w.real(), w.imag()}) {
-      const float hi = (float)c;
-      h.push_back(hi);
-      if (P->rb == 8) h.push_back((float)(c - (ld)hi));
+  h.reserve((size_t)12 << logm);
+  std::vector<std::complex<ld>> w;
+  stage_twiddles(logm, lp, [&](int m) { w.push_back(expi_pi(2 * (int64_t)m, (int64_t)1 << logm)); });
+  for (int s = 1; s <= (P->rb == 8 ? kXfShifts : 1); ++s)
+    for (const auto& x : w) {
+      if (P->rb == 8) {
+        push_xf_twiddle(h, x, s);
+      } else {
+        h.push_back((float)x.real());
+        h.push_back((float)x.imag());
+      }
     }
-  });
   void* d = nullptr;
   PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(float), 16)));
   PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
@@ -1184,6 +1188,12 @@ static int make_fast_args(const pfgb_plan* P, const Pass& ps, const void* in, vo
       // fx: multiply by the significand, add the exponent at the conversion
       F.scale_fx = (long long)llroundl(mant * std::ldexp((ld)1, 60));
       F.emax_shift = k;
+    } else {
+      const ld c = mant * std::ldexp((ld)1, 31);
+      F.scale_xw = (int)std::min<long long>((long long)llroundl(c), 0x7FFFFFFFll);
+      F.scale_xo = (float)std::ldexp(c - (ld)F.scale_xw, -32);
+      F.scale_xf = (float)(mant / 2);
+      F.scale_xe = k + 1;
     }
   }
   if (ps.half_fold && fxi < 0) F.emax_shift -= 1;

@@ -1,0 +1,259 @@
+// Integer-float pairs ("xf"): the arithmetic of the register stages of
+// Float64 (double-float) lines.
+//
+// A double-float (dd) sum costs eight FP32 instructions, and sums are most
+// of an FFT.  Inside the stages of one line a value is held as h + l instead:
+// h a 32-bit integer count of the line's unit q, l a float holding the
+// fraction below it (|l| of a few units).  Sums are one integer and one float
+// addition, exact in h.  A product with a twiddle w, |w| <= 1, is a 32 x 32
+// -> 64-bit integer product with W = round(w 2^(32 - s)): its high word is the
+// new h, in units 2^s q, its low word the new fraction; the rest of w (o =
+// w 2^(32 - s) - W) and the product of l go into the fraction in float.
+//
+// Range: the line's complex values stay within 2^27.5 units in modulus before
+// a radix-8 butterfly and so within 2^30.5 after it: h cannot overflow.  The
+// line enters with components below 2^27 (its largest in [2^26, 2^27)), and
+// the twiddles of each later stage carry the shift s = 1, 2 or 3 that the
+// line's largest component after the previous butterfly asks for
+// (xf_stage_shift; s = 3 always suffices).  The tables hold all three forms,
+// so the shift costs no instruction.
+//
+// Cost: 205 to 265 instructions a point in a 512-point pass, where the dd
+// stages took 277 to 383; 512^3 Float64 round trip 4.14 -> 3.45 ms, 256^3
+// complex 0.945 -> 0.755 ms.
+//
+// Precision: each operation rounds the fraction at about 2^-25 unit, and the
+// line's largest value stays near 2^26 units or above, whatever the data (a
+// fixed s = 3 would leave lines of few non-zero points, which do not grow, at
+// 2^-45).
+#pragma once
+
+#include <stdint.h>
+#include <string.h>
+
+#include "pfgb_dd.cuh"
+#if defined(__CUDACC__)
+#include "pfgb_device.cuh"
+#endif
+
+namespace pfgb {
+
+struct xf {
+  int h;
+  float l;
+  xf() = default;
+  PFGB_HD constexpr xf(int hh, float ll) : h(hh), l(ll) {}
+  // a constant c in (0.5, 1.5), the right-hand operand of a product:
+  // c = 1 + (h + l) 2^-32
+  PFGB_HD constexpr explicit xf(double c)
+      : h((int)((c - 1.0) * 4294967296.0)),
+        l((float)((c - 1.0) * 4294967296.0 - (double)(int)((c - 1.0) * 4294967296.0))) {}
+};
+
+PFGB_HD xf operator+(xf a, xf b) { return xf(a.h + b.h, f_add(a.l, b.l)); }
+PFGB_HD xf operator-(xf a, xf b) { return xf(a.h - b.h, f_sub(a.l, b.l)); }
+PFGB_HD xf operator-(xf a) { return xf(-a.h, -a.l); }
+
+// u 2^-32 + f - 1/2 for the low word u of a product whose high word was rounded
+PFGB_HD float xf_frac(uint32_t u, float f) {
+#if defined(__CUDA_ARCH__)
+  return f_fma(__uint2float_rn(u), 0x1p-32f, f);
+#else
+  return f_fma((float)u, 0x1p-32f, f);
+#endif
+}
+PFGB_HD float xf_i2f(int x) {
+#if defined(__CUDA_ARCH__)
+  return __int2float_rn(x);
+#else
+  return (float)x;
+#endif
+}
+
+// a c, in a's unit
+PFGB_HD xf operator*(xf a, xf c) {
+  const float cf = f_fma((float)c.h, 0x1p-32f, 1.0f);
+  const uint64_t p = 0x80000000u + (uint64_t)((int64_t)a.h * c.h);
+  const float f = f_fma(xf_i2f(a.h), c.l * 0x1p-32f, f_fma(a.l, cf, -0.5f));
+  return xf(a.h + (int)(p >> 32), xf_frac((uint32_t)p, f));
+}
+
+// a c for a factor c in [1/2, 1) given as w = round(c 2^31), o = (c 2^31 - w)
+// 2^-32 and f = c / 2, in units 2 times larger (the ldiv! normalisation).
+PFGB_HD xf xf_scaled(xf a, int w, float o, float f) {
+  const uint64_t p = 0x80000000u + (uint64_t)((int64_t)a.h * w);
+  return xf((int)(p >> 32), xf_frac((uint32_t)p, f_fma(xf_i2f(a.h), o, f_fma(a.l, f, -0.5f))));
+}
+
+// Table entry of a twiddle w for the shift s: round(w 2^(32 - s)) (clamped to
+// 31 bits) and the rest, per part.
+struct xf_tw {
+  int wr, wi;
+  float orr, oi;
+};
+
+// shifts 1 .. kXfShifts: one table each, one after the other
+constexpr int kXfShifts = 3;
+// appends the entry of w (parts of magnitude at most 1, of any precision) for
+// the shift s to a table of 32-bit words
+template <typename V, typename C>
+inline void push_xf_twiddle(V& t, const C& w, int s) {
+  const auto x = w.real(), y = w.imag();
+  const double q = (double)(1ll << (32 - s));
+  const double c[2] = {(double)x * q, (double)y * q};
+  const double rest[2] = {(double)(x - (double)x) * q, (double)(y - (double)y) * q};
+  float o[2];
+  for (int i = 0; i < 2; ++i) {
+    const long long r = (long long)(c[i] < 0 ? c[i] - 0.5 : c[i] + 0.5);
+    const int n = (int)(r > 0x7FFFFFFFll ? 0x7FFFFFFFll : r < -0x7FFFFFFFll ? -0x7FFFFFFFll : r);
+    float f;
+    memcpy(&f, &n, sizeof f);
+    t.push_back(f);
+    o[i] = (float)((c[i] - n) + rest[i]);
+  }
+  t.push_back(o[0]);
+  t.push_back(o[1]);
+}
+
+// (re, im) times w (CONJ: times its conjugate), in units 2^s times larger.
+template <bool CONJ>
+PFGB_HD void xf_twiddle(xf& re, xf& im, xf_tw w) {
+  const int wi = CONJ ? -w.wi : w.wi, mwi = CONJ ? w.wi : -w.wi;
+  const float oi = CONJ ? -w.oi : w.oi;
+  const uint64_t half = 0x80000000u;
+  const uint64_t pr = half + (uint64_t)((int64_t)re.h * w.wr) + (uint64_t)((int64_t)im.h * mwi);
+  const uint64_t pi = half + (uint64_t)((int64_t)re.h * wi) + (uint64_t)((int64_t)im.h * w.wr);
+  const float wrf = xf_i2f(w.wr), wif = xf_i2f(wi), hr = xf_i2f(re.h), hi = xf_i2f(im.h);
+  const float ar = f_fma(re.l, wrf, f_fma(-im.l, wif, f_fma(-hi, oi, f_mul(hr, w.orr))));
+  const float ai = f_fma(re.l, wif, f_fma(im.l, wrf, f_fma(hi, w.orr, f_mul(hr, oi))));
+  re = xf((int)(pr >> 32), xf_frac((uint32_t)pr, f_fma(ar, 0x1p-32f, -0.5f)));
+  im = xf((int)(pi >> 32), xf_frac((uint32_t)pi, f_fma(ai, 0x1p-32f, -0.5f)));
+}
+
+// a in units 2^s times larger
+PFGB_HD xf xf_shift(xf a, int s) {
+#if defined(__CUDA_ARCH__)
+  const float f = __uint_as_float((unsigned)(127 - s) << 23);
+#else
+  const float f = 1.0f / (float)(1 << s);
+#endif
+  return xf(a.h >> s, f_mul(f, f_add(a.l, xf_i2f(a.h & ((1 << s) - 1)))));
+}
+
+// Shift of the twiddles before a butterfly of radix 2^lr, from the line's
+// largest h or ~h: components below 2^(30 - lr) units afterwards, so that the
+// butterfly's sums stay below 2^31 (complex moduli sqrt 2 times the
+// components'), within 1 .. 3.  With 31 bits (moduli up to 2^30.5) three are
+// enough.  A line that keeps one more bit free passes lr + 1.
+PFGB_HD int xf_stage_shift(unsigned m, int lr) {
+#if defined(__CUDA_ARCH__)
+  const int bl = 32 - __clz((int)m);
+#else
+  const int bl = m ? 32 - __builtin_clz(m) : 0;
+#endif
+  const int s = bl - (30 - lr);
+  return s < 1 ? 1 : s > kXfShifts ? kXfShifts : s;
+}
+
+// A dd line in xf units: from the float bits m of its largest |high part|, the
+// scale 2^(153 - e), e the biased exponent of m, at least 27 (a line below
+// 2^-100 keeps fewer bits, as its dd low parts do), that takes the largest
+// component to [2^26, 2^27).  A NaN or an infinity among the high parts gives
+// a NaN (or infinite) fraction, which every sum carries to all of the line.
+PFGB_HD unsigned xf_line_exp(unsigned m) {
+  const unsigned e = m >> 23;
+  return e < 27u ? 27u : e;
+}
+
+#if defined(__CUDACC__)
+__device__ __forceinline__ float xf_scale_in(unsigned e) {
+  return __uint_as_float((280u - e) << 23);
+}
+// biased float exponent of the unit in the dd line's scale, before any shift
+__device__ __forceinline__ unsigned xf_unit_exp(unsigned e) { return min(e, 254u) - 26u; }
+
+__device__ __forceinline__ xf dd2xf(dd a, float f) {
+  const float hs = f_mul(a.h, f);
+  const int h = __float2int_rn(hs);
+  return xf(h, f_fma(a.l, f, f_sub(hs, __int2float_rn(h))));
+}
+// a as the unevaluated sum hi + lo, hi = h rounded to float
+__device__ __forceinline__ void xf_split(xf a, float& hi, float& lo) {
+  hi = __int2float_rn(a.h);
+  lo = f_add(a.l, __int2float_rn(a.h - __float2int_rn(hi)));
+}
+// a 2^(ue - 127): ue the unit's biased exponent
+__device__ __forceinline__ dd xf2dd(xf a, unsigned ue) {
+  const float g = __uint_as_float(ue << 23);
+  float hi, lo;
+  xf_split(a, hi, lo);
+  return dd(f_mul(hi, g), f_mul(lo, g));
+}
+
+// x as a count of 2^(emax - 1023 - B) (B <= 26 bits; emax: the line's largest
+// biased exponent), fs = xf_frac_scale(emax): the 53-bit significand shifted
+// right in 64 bits, its low word as the fraction.  Zeros and subnormals give
+// zero; a line with a NaN or an infinity gets NaN fractions.  No branch, where
+// the conversion to dd needs one for its rare cases.
+__device__ __forceinline__ float xf_frac_scale(int emax) {
+  return __uint_as_float(emax >= 0x7FF ? 0x7FC00000u : 0x2F800000u);  // 2^-32
+}
+template <int B>
+__device__ __forceinline__ xf d2xf(double x, int emax, float fs) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned hi32 = (unsigned)(b >> 32), lo32 = (unsigned)b;
+  const int e = (int)((hi32 >> 20) & 0x7FF);
+  const unsigned mh = (hi32 & 0xFFFFFu) | 0x100000u;
+  const unsigned long long m = (unsigned long long)__funnelshift_l(lo32, mh, B - 20) << 32 | (lo32 << (B - 20));
+  const unsigned long long f = m >> (e == 0 ? 63 : min(emax - e, 63));
+  const int s = (int)hi32 >> 31;
+  const float l = __uint2float_rn((unsigned)f) * __uint_as_float(__float_as_uint(fs) | (hi32 & 0x80000000u));
+  return xf(((int)(f >> 32) ^ s) - s, l);
+}
+
+// A rare result of xf2d: zero, NaN (a NaN or infinite fraction, overflow).
+static __device__ __noinline__ double xf2d_rare(float s, int off) {
+  const unsigned sb = __float_as_uint(s);
+  const int es = (int)(sb >> 23) & 255;
+  if (es == 255 || es + off >= 0x7FF) return __longlong_as_double(0x7FF8000000000000ll);
+  return __longlong_as_double((long long)((unsigned long long)(sb & 0x80000000u) << 32));
+}
+// (re, im) 2^(off - 896) as doubles (off: the unit's biased exponent plus the
+// line's biased double exponent minus 254), within one unit in the last
+// place.  h + l as s + e with s rounded toward zero, so that e has its sign
+// and counts up from s's bit pattern: s gives the high word and the top three
+// bits of the low one, e in units of the double's last place the other 29.
+__device__ __forceinline__ void xf2d(Cx<xf> x, int off, double& re, double& im) {
+  int lo = max(1 - off, 1), hi = min(2046 - off, 254);
+  if (hi < lo) lo = hi = 512;  // no result in the double range
+  bool ok = true;
+  float sv[2];
+  double r[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    float a, b;
+    xf_split(i ? x.im : x.re, a, b);
+    const float s = __fadd_rz(a, b);
+    const float e = __fsub_rn(b, __fsub_rn(s, a));
+    const unsigned sb = __float_as_uint(s);
+    const unsigned esx = sb & 0x7F800000u;
+    ok = ok && (unsigned)((int)(esx >> 23) - lo) <= (unsigned)(hi - lo);
+    const float sux = __uint_as_float(0x99000000u - max(esx, 52u << 23));  // 2^(179 - es)
+    const unsigned li = (unsigned)min(__float2int_rz(__fmul_rn(fabsf(e), sux)), 0x1FFFFFFF);
+    const unsigned hw = (((unsigned)((int)sb >> 3)) & 0x8FFFFFFFu) + ((unsigned)off << 20);
+    r[i] = __hiloint2double((int)hw, (int)((sb << 29) | li));
+    sv[i] = s;
+  }
+  if (!ok) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int es = (int)(__float_as_uint(sv[i]) >> 23) & 255;
+      if ((unsigned)(es - lo) > (unsigned)(hi - lo)) r[i] = xf2d_rare(sv[i], off);
+    }
+  }
+  re = r[0];
+  im = r[1];
+}
+#endif
+
+}  // namespace pfgb

@@ -19,10 +19,10 @@
 // so the shift costs no instruction.
 //
 // Cost: 205 to 265 instructions a point in a 512-point pass, where the dd
-// stages took 277 to 383; 512^3 Float64 round trip 4.14 -> 3.45 ms, 256^3
-// complex 0.945 -> 0.755 ms.
+// stages took 277 to 383; 512^3 Float64 round trip 4.14 -> 3.35 ms, 256^3
+// complex 0.945 -> 0.741 ms.
 //
-// Precision: each operation rounds the fraction at about 2^-25 unit, and the
+// Precision: each operation rounds the fraction at about 2^-24 unit, and the
 // line's largest value stays near 2^26 units or above, whatever the data (a
 // fixed s = 3 would leave lines of few non-zero points, which do not grow, at
 // 2^-45).
@@ -54,7 +54,9 @@ PFGB_HD xf operator+(xf a, xf b) { return xf(a.h + b.h, f_add(a.l, b.l)); }
 PFGB_HD xf operator-(xf a, xf b) { return xf(a.h - b.h, f_sub(a.l, b.l)); }
 PFGB_HD xf operator-(xf a) { return xf(-a.h, -a.l); }
 
-// u 2^-32 + f - 1/2 for the low word u of a product whose high word was rounded
+// u 2^-32 + f for the low word u of a product whose high word was rounded down
+// (to nearest, the rounding constant would cost register moves: 512^3 Float64
+// 3.46 against 3.35 ms)
 PFGB_HD float xf_frac(uint32_t u, float f) {
 #if defined(__CUDA_ARCH__)
   return f_fma(__uint2float_rn(u), 0x1p-32f, f);
@@ -73,16 +75,16 @@ PFGB_HD float xf_i2f(int x) {
 // a c, in a's unit
 PFGB_HD xf operator*(xf a, xf c) {
   const float cf = f_fma((float)c.h, 0x1p-32f, 1.0f);
-  const uint64_t p = 0x80000000u + (uint64_t)((int64_t)a.h * c.h);
-  const float f = f_fma(xf_i2f(a.h), c.l * 0x1p-32f, f_fma(a.l, cf, -0.5f));
+  const uint64_t p = (uint64_t)((int64_t)a.h * c.h);
+  const float f = f_fma(xf_i2f(a.h), c.l * 0x1p-32f, f_mul(a.l, cf));
   return xf(a.h + (int)(p >> 32), xf_frac((uint32_t)p, f));
 }
 
 // a c for a factor c in [1/2, 1) given as w = round(c 2^31), o = (c 2^31 - w)
 // 2^-32 and f = c / 2, in units 2 times larger (the ldiv! normalisation).
 PFGB_HD xf xf_scaled(xf a, int w, float o, float f) {
-  const uint64_t p = 0x80000000u + (uint64_t)((int64_t)a.h * w);
-  return xf((int)(p >> 32), xf_frac((uint32_t)p, f_fma(xf_i2f(a.h), o, f_fma(a.l, f, -0.5f))));
+  const uint64_t p = (uint64_t)((int64_t)a.h * w);
+  return xf((int)(p >> 32), xf_frac((uint32_t)p, f_fma(xf_i2f(a.h), o, f_mul(a.l, f))));
 }
 
 // Table entry of a twiddle w for the shift s: round(w 2^(32 - s)) (clamped to
@@ -120,14 +122,13 @@ template <bool CONJ>
 PFGB_HD void xf_twiddle(xf& re, xf& im, xf_tw w) {
   const int wi = CONJ ? -w.wi : w.wi, mwi = CONJ ? w.wi : -w.wi;
   const float oi = CONJ ? -w.oi : w.oi;
-  const uint64_t half = 0x80000000u;
-  const uint64_t pr = half + (uint64_t)((int64_t)re.h * w.wr) + (uint64_t)((int64_t)im.h * mwi);
-  const uint64_t pi = half + (uint64_t)((int64_t)re.h * wi) + (uint64_t)((int64_t)im.h * w.wr);
+  const uint64_t pr = (uint64_t)((int64_t)re.h * w.wr) + (uint64_t)((int64_t)im.h * mwi);
+  const uint64_t pi = (uint64_t)((int64_t)re.h * wi) + (uint64_t)((int64_t)im.h * w.wr);
   const float wrf = xf_i2f(w.wr), wif = xf_i2f(wi), hr = xf_i2f(re.h), hi = xf_i2f(im.h);
   const float ar = f_fma(re.l, wrf, f_fma(-im.l, wif, f_fma(-hi, oi, f_mul(hr, w.orr))));
   const float ai = f_fma(re.l, wif, f_fma(im.l, wrf, f_fma(hi, w.orr, f_mul(hr, oi))));
-  re = xf((int)(pr >> 32), xf_frac((uint32_t)pr, f_fma(ar, 0x1p-32f, -0.5f)));
-  im = xf((int)(pi >> 32), xf_frac((uint32_t)pi, f_fma(ai, 0x1p-32f, -0.5f)));
+  re = xf((int)(pr >> 32), xf_frac((uint32_t)pr, f_mul(ar, 0x1p-32f)));
+  im = xf((int)(pi >> 32), xf_frac((uint32_t)pi, f_mul(ai, 0x1p-32f)));
 }
 
 // a in units 2^s times larger

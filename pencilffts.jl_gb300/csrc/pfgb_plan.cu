@@ -628,8 +628,12 @@ static int upload_tc_table(pfgb_plan* P, int logm, int sign, const void** out) {
   return PFGB_OK;
 }
 
-// Radix plan for a DFT length: returns false if a prime factor > 13 remains.
+// Radix plan for a DFT length of the generic kernel: returns false if a prime
+// factor > 13 remains, or if a stage has more butterflies than a block has
+// threads (the stages run in place, one butterfly a thread).
+constexpr int kMaxButterflies = 1024;
 static bool factor_radices(int n, std::vector<int>& rad) {
+  const int len = n;
   rad.clear();
   int e = 0;
   while (n % 2 == 0) { n /= 2; ++e; }
@@ -646,7 +650,7 @@ static bool factor_radices(int n, std::vector<int>& rad) {
     }
   }
   for (int p : odds) rad.push_back(p);
-  return true;
+  return rad.empty() || len / *std::min_element(rad.begin(), rad.end()) <= kMaxButterflies;
 }
 
 // ---------------------------------------------------------------------------

@@ -168,3 +168,13 @@ def test_long_lines_in_a_batch(cuda):
             assert rel(v.to_logical(), oracle_plan(p).forward(x)) <= 1e-5
             assert rel(w.to_logical(), x) <= 1e-5
         assert b.status() == 0
+
+
+@pytest.mark.parametrize("real", [F64, F32])
+@pytest.mark.parametrize("n", [2050, 3456, 4050, 6174])
+def test_lines_of_many_butterflies(cuda, real, n):
+    """Lengths whose smallest radix leaves a stage more butterflies than a
+    block has threads, and the R2R lines whose extension is such a length."""
+    for tr in (T.FFT(), T.RFFT(), T.R2R(2)):
+        check_plan(P.PencilFFTPlan((n,), tr, real, extra_dims=(3,)), seed=n)
+    check_plan(P.PencilFFTPlan((n // 2,), T.R2R(5), real, extra_dims=(3,)), seed=n)

@@ -28,6 +28,12 @@
 
 namespace pfgb {
 
+// Smooth-length pass (sm_pass): stages and lines of a tile at most, and its
+// largest shared memory
+constexpr int kSmStages = 6;
+constexpr int kSmLines = 64;
+constexpr int kSmMaxSmem = 200 * 1024;
+
 struct FastArgs {
   const void* in;
   void* out;
@@ -41,6 +47,13 @@ struct FastArgs {
   const void* bs_chirp;
   const void* bs_filt;
   Div31 div_m;
+  // smooth-length pass (sm_pass): line length, lines of a tile, pitch of a
+  // line in shared memory, stages with their radix, first twiddle entry and
+  // sub-length, entries of one twiddle table, divisors by the points of an
+  // input and of an output line
+  int sm_m, sm_tw, sm_pitch, sm_nst, sm_ntw;
+  int sm_r[kSmStages], sm_tw0[kSmStages];
+  Div31 sm_ls[kSmStages], sm_din, sm_dout;
   // OP_C2CT (first pass of a split line of M = M1 * M2 points): outputs times
   // exp(sign 2 pi i n1 k2 / M) from t4_tab (M entries), n1 the index along
   // the dimension of role t4_role (1 tile, 2 + o outer)

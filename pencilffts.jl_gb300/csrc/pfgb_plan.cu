@@ -124,6 +124,9 @@ struct Pass {
   bool mr = false;
   int r0 = 0, logn = 0;
   const void* ftw2 = nullptr;  // its other twiddles (upload_mr_table); tensor-core form: the M-point table
+  // smooth-length pass (sm_pass): radices, butterfly step of a thread
+  bool sm = false;
+  int sm_nst = 0, sm_r[kSmStages] = {};
   // Bluestein register pass (bs_pass) for other lines up to 2048 points:
   // convolution length 2^logl (ftw holds its twiddles), chirp and filter
   // tables; the generic kernel's geometry is kept (g_*) for executions it
@@ -721,7 +724,7 @@ static int bluestein_form(pfgb_plan* P, Pass& ps) {
   if (!rc) rc = upload_fast_vec(P, "bsw" + key, w, &ps.bs_chirp);
   if (!rc) rc = upload_fast_vec(P, "bsf" + key, bf, &ps.bs_filt);
   if (rc) return rc;
-  ps.mr = false;
+  ps.mr = ps.sm = false;
   ps.fast = false;
   ps.bs = true;
   ps.fop = ps.op;
@@ -731,6 +734,132 @@ static int bluestein_form(pfgb_plan* P, Pass& ps) {
   ps.lines = pk ? 2 * ps.clines : ps.clines;
   ps.threads = P->rb == 8 ? bs_threads<dd>(logl) : bs_threads<float>(logl);
   ps.smem = P->rb == 8 ? bs_smem<dd>(logl) : bs_smem<float>(logl);
+  return PFGB_OK;
+}
+
+static int tile_dim(const Pass& ps);
+// Radices of a smooth length M for the smooth-length pass: fewest stages, then
+// the smallest sum; false if M has another factor.
+static bool sm_radices(int M, bool f64, int& nst, int (&r)[kSmStages]) {
+  static const int all[] = {16, 15, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  int cur[kSmStages], best_n = kSmStages + 1, best_sum = 0;
+  auto search = [&](auto&& self, int m, int depth, int from, int sum) -> void {
+    if (m == 1) {
+      if (depth < best_n || (depth == best_n && sum < best_sum)) {
+        best_n = depth;
+        best_sum = sum;
+        for (int i = 0; i < depth; ++i) r[i] = cur[i];
+      }
+      return;
+    }
+    if (depth >= kSmStages || depth >= best_n) return;
+    for (int i = from; i < (int)(sizeof(all) / sizeof(all[0])); ++i) {
+      if (f64 && all[i] > 8) continue;
+      if (m % all[i]) continue;
+      cur[depth] = all[i];
+      self(self, m / all[i], depth + 1, i, sum + all[i]);
+    }
+  };
+  search(search, M, 0, 0, 0);
+  nst = best_n;
+  return best_n <= kSmStages;
+}
+
+// The smooth-length form of a c2c / r2c / c2r pass of ps.M points (2, 3, 5 and
+// 7 only): radices, lines of a tile and threads, twiddle tables; taken = false
+// if the pass does not take it.  It takes every length that has no
+// power-of-two form, on Float64 data also those of the mixed-radix pass
+// (3 or 5 times a power of two; its Float32 form stays the faster one: 384^3
+// 0.85 ms, where 360^3 takes 0.93 here), with 16 complex lines or more.  Fewer
+// lines keep the Bluestein or mixed-radix tile where those have the length
+// (few): launch latency sets their time, and the plans that ask for those
+// kernels by name in tests have few lines.  Measured round trips, Bluestein or
+// (*) mixed-radix tile against this one: Float64 RFFT 100^3 0.213 -> 0.088 ms,
+// 240^3 1.98 -> 0.67, 360^3 9.73 -> 2.6, *384^3 3.97 -> 2.79, FFT *96^3 0.286
+// -> 0.100, *24^3 0.139 -> 0.045, 1000^2 0.260 -> 0.133, 3000^2 (generic
+// kernel) 4.27 -> 0.96; Float32 RFFT 360^3 3.45 -> 0.93, 120^3 0.088 -> 0.069,
+// 50x60x70 0.040 -> 0.041, FFT 200^3 0.629 -> 0.298.
+//
+// The tile: w lines and a butterfly step q (w q threads), by the share of
+// threads that have work in every stage, the threads in flight on an SM, 64
+// contiguous bytes at least on a strided axis, 8 lines side by side for the
+// banks, and the last wave.
+static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
+  taken = false;
+  const int M = ps.M;
+  const bool f64 = P->rb == 8, pk = fast_packed(ps.op);
+  int nst = 0, r[kSmStages];
+  if (M < 6 || M > 4096 || !sm_radices(M, f64, nst, r)) return PFGB_OK;
+  // lines along the tile dimension and outside it
+  const int td = tile_dim(ps);
+  const int64_t nt = td >= 0 ? ps.lin.size[td] : 1, ncl = pk ? (nt + 1) / 2 : nt;
+  int64_t outer = 1;
+  for (int d = 0; d < ps.lin.D; ++d)
+    if (d != ps.axis && d != td) outer *= ps.lin.size[d];
+  if (ncl * outer < 16 && !few) return PFGB_OK;
+  const bool strided = ps.lin.perm[0] != ps.axis || ps.lout.perm[0] != ps.axis;
+  const int pitch = (M + 2) | 1, ebytes = f64 ? 16 : 8;
+  double best = 1e30;
+  int tw = 0, k = 0;
+  for (int w = 1; w <= kSmLines && w <= std::max<int64_t>(ncl, 1); ++w) {
+    const size_t smem = (size_t)2 * w * pitch * ebytes;
+    if (smem > (size_t)kSmMaxSmem) break;
+    for (int q = 1; q * w <= 256; ++q) {
+      const int threads = q * w, warps = (threads + 31) / 32;
+      double points = 0;  // a thread's points over the stages
+      bool useful = false;
+      for (int s = 0; s < nst; ++s) {
+        const int T = M / r[s];
+        points += r[s] * ((T + q - 1) / q);
+        useful = useful || T % q == 0 || q < T;
+      }
+      if (!useful) continue;
+      double cost = points * warps * 32 / ((double)w * M * nst);  // idle lanes
+      const int ctas = (int)std::min<size_t>({(size_t)227 * 1024 / (smem + 3072), (size_t)(f64 ? 24 : 32) / warps, (size_t)32});
+      if (ctas < 1) continue;
+      const double occ = (double)ctas * threads;  // threads in flight on an SM
+      if (occ < 768) cost *= std::sqrt(768 / occ);
+      const int chunk = w * 2 * P->rb;  // contiguous bytes on a strided axis
+      if (strided && chunk < 128) cost *= chunk >= 64 ? 1.1 : 1.1 * 64 / chunk;
+      if (w < 8) cost *= 1.2;  // bank conflicts of less than 8 lines side by side
+      const double waves = (double)((ncl + w - 1) / w * outer) / (152.0 * ctas);
+      cost *= std::ceil(waves) / waves * ((double)((ncl + w - 1) / w * w) / ncl);
+      if (cost < best) { best = cost; tw = w; k = q; }
+    }
+  }
+  if (!tw) return PFGB_OK;
+  const std::string key = (f64 ? "smx" : "smf") + std::to_string(M);
+  if (!P->query_only && !P->tables.count(key)) {
+    std::vector<std::complex<ld>> w;
+    for (int s = 1, Ls = r[0]; s < nst; Ls *= r[s], ++s)
+      for (int q = 1; q < r[s]; ++q)
+        for (int j = 0; j < Ls; ++j) w.push_back(expi_pi(2 * (int64_t)q * j, (int64_t)r[s] * Ls));
+    std::vector<float> h;
+    for (int s = 1; s <= (f64 ? kXfShifts : 1); ++s)
+      for (const auto& x : w) {
+        if (f64) {
+          push_xf_twiddle(h, x, s);
+        } else {
+          h.push_back((float)x.real());
+          h.push_back((float)x.imag());
+        }
+      }
+    void* d = nullptr;
+    PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(float), 16)));
+    PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+    P->tables[key] = d;
+  }
+  ps.ftw = P->query_only ? nullptr : P->tables[key];
+  ps.sm = true;
+  ps.mr = ps.bs = ps.fast = false;
+  ps.fop = ps.op;
+  ps.sm_nst = nst;
+  for (int s = 0; s < nst; ++s) ps.sm_r[s] = r[s];
+  ps.clines = tw;
+  ps.lines = pk ? 2 * tw : tw;
+  ps.threads = tw * k;
+  ps.smem = (size_t)2 * tw * pitch * ebytes;
+  taken = true;
   return PFGB_OK;
 }
 
@@ -896,6 +1025,11 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
       if (M % r0) continue;
       const int n = M / r0;
       if (n < 8 || n > 512 || (n & (n - 1))) continue;
+      if (P->rb == 8) {
+        bool smooth = false;
+        rc = sm_form(P, ps, false, smooth);
+        if (rc || smooth) return rc;
+      }
       ps.mr = true;
       ps.fop = ps.op;
       ps.r0 = r0;
@@ -938,6 +1072,15 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
   if (ps.smem > 200 * 1024)
     return fail(PFGB_ERR_UNSUPPORTED, "line does not fit in shared memory");
   ps.zero_fill = ps.L > 0 || (ps.op == OP_R2R_C || ps.op == OP_R2R_R);
+  // other c2c / r2c / c2r lines of 2, 3, 5 and 7 only take the smooth-length
+  // pass (integer-float for Float64 data unless native FP64 was requested;
+  // Float64 lines above 2048 points stay in FP64, which is more precise)
+  if ((ps.op == OP_C2C || ps.op == OP_R2C || ps.op == OP_C2R) &&
+      !(P->rb == 8 && (P->precision == PFGB_PRECISION_NATIVE || M > 2048))) {
+    bool smooth = false;
+    rc = sm_form(P, ps, M > 2048, smooth);
+    if (rc || smooth) return rc;
+  }
   // other c2c / r2c / c2r lines up to 2048 points take the Bluestein register
   // pass (double-float for Float64 data unless native FP64 was requested)
   if ((ps.op == OP_C2C || ps.op == OP_R2C || ps.op == OP_C2R) && M >= 2 && M <= 2048 &&
@@ -1209,6 +1352,23 @@ static int make_fast_args(const pfgb_plan* P, const Pass& ps, const void* in, vo
     F.te_rescale = 0;
     F.te = nullptr;
   }
+  if (ps.sm) {
+    F.sm_m = ps.M;
+    F.sm_tw = ps.clines;
+    F.sm_pitch = (ps.M + 2) | 1;
+    F.sm_nst = ps.sm_nst;
+    int Ls = 1, at = 0;
+    for (int s = 0; s < ps.sm_nst; ++s) {
+      F.sm_r[s] = ps.sm_r[s];
+      F.sm_tw0[s] = at;
+      F.sm_ls[s] = make_div31(Ls);
+      if (s > 0) at += (ps.sm_r[s] - 1) * Ls;
+      Ls *= ps.sm_r[s];
+    }
+    F.sm_ntw = at;
+    F.sm_din = make_div31(ps.op == OP_C2R ? ps.M / 2 + 1 : ps.M);
+    F.sm_dout = make_div31(ps.op == OP_R2C ? ps.M / 2 + 1 : ps.M);
+  }
   if (A.nterm > 0) {
     if (ps.fop != OP_C2C) return fail(PFGB_ERR_UNSUPPORTED, "internal: derivative sum on a non-c2c pass");
     F.op = OP_CSUM;
@@ -1368,6 +1528,19 @@ static Pass generic_form(const Pass& ps) {
 
 // mixed-radix pass of a plan (grid == 0: configure only); OP_CSUM runs the
 // c2c kernel (its load sums the terms)
+int launch_sm_f32_c2c(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
+int launch_sm_f32_r2c(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
+int launch_sm_f32_c2r(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
+int launch_sm_dd_c2c(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
+int launch_sm_dd_r2c(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
+int launch_sm_dd_c2r(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
+static int launch_sm(const pfgb_plan* P, const Pass& ps, const FastArgs& F, int64_t grid, cudaStream_t s) {
+  const bool d = P->rb == 8;
+  const auto f = ps.op == OP_C2C ? (d ? launch_sm_dd_c2c : launch_sm_f32_c2c)
+                 : ps.op == OP_R2C ? (d ? launch_sm_dd_r2c : launch_sm_f32_r2c)
+                                   : (d ? launch_sm_dd_c2r : launch_sm_f32_c2r);
+  return f(ps.sign, F, grid, ps.threads, ps.smem, s);
+}
 static int launch_mr(const pfgb_plan* P, const Pass& ps, const FastArgs& F, int64_t grid, cudaStream_t s) {
   const bool d = P->rb == 8;
   switch (F.op) {
@@ -2060,12 +2233,12 @@ static int execute(pfgb_plan* P, const Direction& dir, void* dst, const void* sr
         rc = launch_plain(P, ps, F, grid, s);
       }
       if (rc) return rc;
-    } else if (ps.mr) {
+    } else if (ps.mr || ps.sm) {
       FastArgs F;
       int64_t grid = 0;
       int rc = make_fast_args(P, ps, in, out, normalise && i == last_tr, F, grid, i == dpass ? dv : nullptr);
       if (rc) return rc;
-      rc = launch_mr(P, ps, F, grid, s);
+      rc = ps.sm ? launch_sm(P, ps, F, grid, s) : launch_mr(P, ps, F, grid, s);
       if (rc) return rc;
     } else if (ps.bs && ps.variant != 2 && !(i == dpass && dv && dv->mode == 3)) {
       FastArgs F;
@@ -2861,6 +3034,10 @@ static int plan_build(const pfgb_plan_desc* desc, pfgb_plan** out, bool query_on
           std::memset(&F, 0, sizeof(F));
           F.op = ps.fop;
           rc = launch_mr(P, ps, F, 0, nullptr);
+        } else if (ps.sm) {
+          FastArgs F;
+          std::memset(&F, 0, sizeof(F));
+          rc = launch_sm(P, ps, F, 0, nullptr);
         } else if (ps.bs) {
           FastArgs F;
           std::memset(&F, 0, sizeof(F));
@@ -3163,6 +3340,7 @@ int pfgb_plan_get_timing(pfgb_plan* P, pfgb_pass_timing* out, int max, int* n) {
                         : ps.variant == 1 ? (P->rb == 8 ? "fast_pass_tma<dd>" : "fast_pass_tma<float>")
                         : ps.fast ? (P->rb == 4 ? "fast_pass<float>" : P->fx ? "fast_pass<fx>" : "fast_pass<dd>")
                         : ps.mr ? (P->rb == 4 ? "mr_pass<float>" : "mr_pass<dd>")
+                        : ps.sm ? (P->rb == 4 ? "sm_pass<float>" : "sm_pass<dd>")
                         : ps.bs && ps.variant != 2 ? (P->rb == 4 ? "bs_pass<float>" : "bs_pass<dd>")
                                   : (P->rb == 8 ? "pass_kernel<double>" : "pass_kernel<float>");
     std::snprintf(e.kernel, sizeof(e.kernel), "%s", kname);

@@ -1,0 +1,13 @@
+// Smooth-length pass, integer-float pairs for Float64 data, c2r lines.
+#include <cuda_runtime.h>
+
+#include "pencilfft_gb300.h"
+#include "pfgb_sm.cuh"
+
+namespace pfgb {
+
+int launch_sm_dd_c2r(int, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s) {
+  return launch_sm_one<xf, 1, OP_C2R>(A, grid, threads, smem, s);
+}
+
+}  // namespace pfgb

@@ -33,6 +33,17 @@ namespace pfgb {
 constexpr int kSmStages = 6;
 constexpr int kSmLines = 64;
 constexpr int kSmMaxSmem = 200 * 1024;
+// How it takes an R2R line of n points:
+//   D2 (REDFT10, RODFT10, DHT): the n-point DFT V of the line (REDFT10 / RODFT10:
+//      even points first, odd ones backwards after them), then
+//      Y[k] = w_k V[k] + conj(w_k) V[n - k], w_k = exp(-i pi k / (2n)) (DHT: (1 + i) / 2)
+//   D3 (REDFT01, RODFT01): the inverse steps in the opposite order
+//   X (REDFT00, RODFT00): the DFT of the even / odd extension, 2 (n -+ 1) points
+//   D4 (REDFT11, RODFT11): the 2n-point DFT of the line and its mirror image
+//      times c_j = exp(-i pi j / (2n)), then Y[k] = d_k V[k], d_k = exp(-i pi (2k + 1) / (4n))
+// RODFT kinds are the REDFT ones with points negated or reversed (D2, D3) or
+// an odd mirror image; all hold for complex lines, so two real lines travel as one.
+enum SmMode { SM_D2 = 0, SM_D3 = 1, SM_X = 2, SM_D4 = 3 };
 
 struct FastArgs {
   const void* in;
@@ -54,6 +65,7 @@ struct FastArgs {
   int sm_m, sm_tw, sm_pitch, sm_nst, sm_ntw;
   int sm_r[kSmStages], sm_tw0[kSmStages];
   Div31 sm_ls[kSmStages], sm_din, sm_dout;
+  int sm_mode;  // R2R lines: SmMode
   // OP_C2CT (first pass of a split line of M = M1 * M2 points): outputs times
   // exp(sign 2 pi i n1 k2 / M) from t4_tab (M entries), n1 the index along
   // the dimension of role t4_role (1 tile, 2 + o outer)

@@ -126,6 +126,7 @@ struct Pass {
   const void* ftw2 = nullptr;  // its other twiddles (upload_mr_table); tensor-core form: the M-point table
   // smooth-length pass (sm_pass): radices, butterfly step of a thread
   bool sm = false;
+  int sm_mode = 0;  // R2R lines (SmMode)
   int sm_nst = 0, sm_r[kSmStages] = {};
   // Bluestein register pass (bs_pass) for other lines up to 2048 points:
   // convolution length 2^logl (ftw holds its twiddles), chirp and filter
@@ -765,6 +766,26 @@ static bool sm_radices(int M, bool f64, int& nst, int (&r)[kSmStages]) {
   return best_n <= kSmStages;
 }
 
+// A table of the smooth-length pass: float (re, im), or xf_tw for Float64 plans,
+// one after the other for the shifts 1 .. shifts.
+static int upload_sm_vec(pfgb_plan* P, const std::string& key, const std::vector<std::complex<ld>>& w, int shifts) {
+  std::vector<float> h;
+  for (int s = 1; s <= (P->rb == 8 ? shifts : 1); ++s)
+    for (const auto& x : w) {
+      if (P->rb == 8) {
+        push_xf_twiddle(h, x, s);
+      } else {
+        h.push_back((float)x.real());
+        h.push_back((float)x.imag());
+      }
+    }
+  void* d = nullptr;
+  PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(float), 16)));
+  P->tables[key] = d;
+  PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+  return PFGB_OK;
+}
+
 // The smooth-length form of a c2c / r2c / c2r pass of ps.M points (2, 3, 5 and
 // 7 only): radices, lines of a tile and threads, twiddle tables; taken = false
 // if the pass does not take it.  It takes every length that has no
@@ -787,7 +808,7 @@ static bool sm_radices(int M, bool f64, int& nst, int (&r)[kSmStages]) {
 static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
   taken = false;
   const int M = ps.M;
-  const bool f64 = P->rb == 8, pk = fast_packed(ps.op);
+  const bool f64 = P->rb == 8, pk = fast_packed(ps.op) || ps.op == OP_R2R_R;
   int nst = 0, r[kSmStages];
   if (M < 6 || M > 4096 || !sm_radices(M, f64, nst, r)) return PFGB_OK;
   // lines along the tile dimension and outside it
@@ -834,22 +855,11 @@ static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
     for (int s = 1, Ls = r[0]; s < nst; Ls *= r[s], ++s)
       for (int q = 1; q < r[s]; ++q)
         for (int j = 0; j < Ls; ++j) w.push_back(expi_pi(2 * (int64_t)q * j, (int64_t)r[s] * Ls));
-    std::vector<float> h;
-    for (int s = 1; s <= (f64 ? kXfShifts : 1); ++s)
-      for (const auto& x : w) {
-        if (f64) {
-          push_xf_twiddle(h, x, s);
-        } else {
-          h.push_back((float)x.real());
-          h.push_back((float)x.imag());
-        }
-      }
-    void* d = nullptr;
-    PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(float), 16)));
-    PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
-    P->tables[key] = d;
+    const int rc = upload_sm_vec(P, key, w, kXfShifts);
+    if (rc) return rc;
   }
   ps.ftw = P->query_only ? nullptr : P->tables[key];
+  ps.L = 0;
   ps.sm = true;
   ps.mr = ps.bs = ps.fast = false;
   ps.fop = ps.op;
@@ -860,6 +870,57 @@ static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
   ps.threads = tw * k;
   ps.smem = (size_t)2 * tw * pitch * ebytes;
   taken = true;
+  return PFGB_OK;
+}
+
+static bool one_pass_length(int64_t n);
+static int64_t r2r_extension(int kind, int64_t n);
+static bool r2r_register_form(const pfgb_plan* P, int kind, int64_t n);
+// Whether R2R lines of n points take the smooth-length pass, with the mode and
+// the points of its DFT: lengths without a power-of-two form whose DFT length
+// is smooth, on Float64 data where the lines would otherwise go through a
+// gathered extension in double-float (not those of the native-FP64 kernel,
+// which is more precise).
+static bool sm_r2r(const pfgb_plan* P, int kind, int64_t n, int& mode, int& M) {
+  if (P->fx || (P->rb == 8 && P->precision == PFGB_PRECISION_NATIVE) || n < 2 || r2r_register_form(P, kind, n)) return false;
+  const int64_t ext = r2r_extension(kind, n);
+  if (P->rb == 8 && !one_pass_length(ext)) return false;
+  switch (kind) {
+    case K_DHT: case K_REDFT10: case K_RODFT10: mode = SM_D2; break;
+    case K_REDFT01: case K_RODFT01: mode = SM_D3; break;
+    case K_REDFT00: case K_RODFT00: mode = SM_X; break;
+    default: mode = SM_D4; break;
+  }
+  const int64_t m = mode == SM_D2 || mode == SM_D3 ? n : ext;
+  int nst, r[kSmStages];
+  if (m < 6 || m > 4096 || !sm_radices((int)m, P->rb == 8, nst, r)) return false;
+  M = (int)m;
+  return true;
+}
+static int sm_r2r_form(pfgb_plan* P, Pass& ps, int mode, int M) {
+  const int n = (int)ps.lin.size[ps.axis];
+  ps.M = M;
+  ps.sign = -1;
+  ps.sm_mode = mode;
+  bool taken = false;
+  int rc = sm_form(P, ps, true, taken);
+  if (rc) return rc;
+  if (!taken) return fail(PFGB_ERR_UNSUPPORTED, "internal: smooth-length form of an R2R line");
+  const bool dht = ps.r2r_kind == K_DHT;
+  const std::string key = (P->rb == 8 ? "smrx" : "smrf") + std::to_string(mode) + (dht ? "h" : "/") + std::to_string(n);
+  if (P->query_only || mode == SM_X) return PFGB_OK;
+  if (!P->tables.count(key)) {
+    std::vector<std::complex<ld>> w;
+    if (mode == SM_D4) {
+      for (int j = 0; j < 2 * n; ++j) w.push_back(expi_pi(j, 2 * (int64_t)n));
+      for (int k = 0; k < n; ++k) w.push_back(expi_pi(2 * (int64_t)k + 1, 4 * (int64_t)n));
+    } else {
+      for (int k = 0; k < n; ++k) w.push_back(dht ? std::complex<ld>(0.5L, 0.5L) : expi_pi(k, 2 * (int64_t)n));
+    }
+    rc = upload_sm_vec(P, key, w, 1);
+    if (rc) return rc;
+  }
+  ps.d23_tab = P->tables[key];
   return PFGB_OK;
 }
 
@@ -901,6 +962,10 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
   if (n_in > kMaxLc * 2 || n_out > kMaxLc * 2)
     return fail(PFGB_ERR_UNSUPPORTED, "line too long");
   int M = 0;
+  if (ps.op == OP_R2R_C || ps.op == OP_R2R_R) {
+    int mode = 0;
+    if (sm_r2r(P, ps.r2r_kind, n_in, mode, M)) return sm_r2r_form(P, ps, mode, M);
+  }
   switch (ps.op) {
     case OP_C2C: M = (int)n_in; break;
     case OP_R2C: M = (int)n_in; break;
@@ -1366,8 +1431,9 @@ static int make_fast_args(const pfgb_plan* P, const Pass& ps, const void* in, vo
       Ls *= ps.sm_r[s];
     }
     F.sm_ntw = at;
-    F.sm_din = make_div31(ps.op == OP_C2R ? ps.M / 2 + 1 : ps.M);
-    F.sm_dout = make_div31(ps.op == OP_R2C ? ps.M / 2 + 1 : ps.M);
+    F.sm_mode = ps.sm_mode;
+    F.sm_din = make_div31(A.n_in);
+    F.sm_dout = make_div31(A.n_out);
   }
   if (A.nterm > 0) {
     if (ps.fop != OP_C2C) return fail(PFGB_ERR_UNSUPPORTED, "internal: derivative sum on a non-c2c pass");
@@ -1534,8 +1600,12 @@ int launch_sm_f32_c2r(int sign, const FastArgs& A, int64_t grid, int threads, si
 int launch_sm_dd_c2c(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
 int launch_sm_dd_r2c(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
 int launch_sm_dd_c2r(int sign, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
+int launch_sm_f32_r2r(bool cplx, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
+int launch_sm_dd_r2r(bool cplx, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s);
 static int launch_sm(const pfgb_plan* P, const Pass& ps, const FastArgs& F, int64_t grid, cudaStream_t s) {
   const bool d = P->rb == 8;
+  if (ps.op == OP_R2R_C || ps.op == OP_R2R_R)
+    return (d ? launch_sm_dd_r2r : launch_sm_f32_r2r)(ps.op == OP_R2R_C, F, grid, ps.threads, ps.smem, s);
   const auto f = ps.op == OP_C2C ? (d ? launch_sm_dd_c2c : launch_sm_f32_c2c)
                  : ps.op == OP_R2C ? (d ? launch_sm_dd_r2c : launch_sm_f32_r2c)
                                    : (d ? launch_sm_dd_c2r : launch_sm_f32_c2r);
@@ -1849,6 +1919,8 @@ static bool expand_long_r2r(const pfgb_plan* P, const Pass& ps, Pass& pre, Pass&
   const int64_t n = ps.lin.size[a];
   if (n < 2 || ps.lin.D > kMaxOuter) return false;
   const int64_t m = r2r_extension(ps.r2r_kind, n);
+  int mode, dft;
+  if (sm_r2r(P, ps.r2r_kind, n, mode, dft)) return false;
   std::vector<int> rad;
   const bool generic = m <= kMaxLc && (factor_radices((int)m, rad) || bluestein_length(m) <= kMaxLc);
   const int form = long_c2c_form(m);
@@ -2170,7 +2242,10 @@ static int execute(pfgb_plan* P, const Direction& dir, void* dst, const void* sr
   // Float64 fast passes: fx, or dd for an execution with a fused derivative
   const bool fxrun = P->fx && !(dv && dv->mode);
   if (dv && dv->mode) {
-    if (dpass < 0 || dir.passes[dpass].op != OP_C2C)
+    // (Float64 R2R lines of the smooth-length pass along another dimension take
+    // the factor too, as the c2c pass of their gathered extension does)
+    if (dpass < 0 || (dir.passes[dpass].op != OP_C2C &&
+                      !(dir.passes[dpass].op == OP_R2R_C && dir.passes[dpass].sm && P->rb == 8 && dv->mode != 3)))
       return fail(PFGB_ERR_UNSUPPORTED, "the fused derivative needs a complex-to-complex pass at that end "
                                         "of the plan");
     if (dir.passes[dpass].four)

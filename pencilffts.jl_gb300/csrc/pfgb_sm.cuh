@@ -1,6 +1,7 @@
 // Smooth-length pass: lines of M points, M a product of 2, 3, 5 and 7 that no
-// power-of-two pass takes, for c2c, r2c and c2r, any input / output layout, in
-// FP32 or (Float64 data) in integer-float pairs, doubles in and out.
+// power-of-two pass takes, for c2c, r2c, c2r and the R2R kinds (SmMode), any
+// input / output layout, in FP32 or (Float64 data) in integer-float pairs,
+// doubles in and out.
 //
 // A tile of TW lines goes through nst Stockham stages of mixed radix between
 // two shared-memory buffers.  A thread owns one line of the tile (p = thread
@@ -281,9 +282,12 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
   using MC = typename std::conditional<XF, double2, float2>::type;
   // xf: bits of the largest component at the first stage, below 27 by one for
   // the r2c split's sum and for c2r's sum of two spectra
-  constexpr int HEAD = OP == OP_R2C ? 1 : 0;
-  constexpr int BITS = 26 - (OP == OP_C2C ? 0 : 1);
-  constexpr bool packed = OP != OP_C2C;
+  constexpr bool R2R = OP == OP_R2R_C || OP == OP_R2R_R;
+  constexpr bool CIN = OP == OP_C2C || OP == OP_R2R_C;  // complex elements in and out
+  // (D2: for its sum of two outputs; D4: one above, its first twiddles shift by one)
+  const int head = OP == OP_R2C || (R2R && a.sm_mode == SM_D2) ? 1 : 0;
+  const int bits = !R2R ? 26 - (OP == OP_C2C ? 0 : 1) : a.sm_mode == SM_D2 ? 25 : a.sm_mode == SM_D4 ? 27 : 26;
+  constexpr bool packed = !CIN;
   __shared__ unsigned lm[kSmStages][kSmLines];  // xf: per line, the input's largest exponent, then the stages' components
   __shared__ int loff[kSmLines];
   const int TW = a.sm_tw, M = a.sm_m, pitch = a.sm_pitch, NT = blockDim.x, tid = threadIdx.x;
@@ -308,7 +312,7 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
   // real lines' elements
   auto in1 = [&](int i, int64_t off) {
     MC x{0, 0};
-    if constexpr (OP == OP_C2C) {
+    if constexpr (CIN) {
       if (i < nvalid) x = reinterpret_cast<const MC*>(a.in)[off];
     } else {
       const MR* in = reinterpret_cast<const MR*>(a.in) + off;
@@ -318,7 +322,7 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
     return x;
   };
   // with a derivative on the input: i k src, or the sum of i k_t src_t
-  const bool spectral = OP == OP_C2C && (a.nterm > 0 || a.deriv == 1);
+  const bool spectral = CIN && (a.nterm > 0 || a.deriv == 1);
   auto in1k = [&](int i, int pos, int64_t off) {
     MC x{0, 0};
     if (i >= nvalid) return x;
@@ -345,6 +349,32 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
     return x;
   };
   const int m = M / 2 + 1;  // half spectrum of a c2r line
+  const int n = a.n_in, odd = a.r2r_odd;  // R2R lines
+  // where point k of an R2R line goes before a D2 transform, and where it comes
+  // from after a D3 one
+  auto even_odd = [&](int k) { return k & 1 ? n - ((k + 1) >> 1) : k >> 1; };
+  // point k of the array line to the tile's line
+  auto put = [&](MC* zl, int k, MC x) {
+    if constexpr (!R2R) {
+      zl[k] = x;
+    } else if (a.sm_mode == SM_D2) {
+      if (odd == 1 && (k & 1)) x = MC{-x.x, -x.y};
+      zl[odd == 2 ? k : even_odd(k)] = x;
+    } else if (a.sm_mode == SM_D3) {
+      zl[odd ? n - 1 - k : k] = x;
+    } else if (a.sm_mode == SM_X) {
+      if (odd) {
+        zl[k + 1] = x;
+        zl[M - 1 - k] = MC{-x.x, -x.y};
+      } else {
+        zl[k] = x;
+        if (k >= 1 && k <= n - 2) zl[M - k] = x;
+      }
+    } else {
+      zl[k] = x;
+    }
+  };
+  const bool pre = R2R && (a.sm_mode == SM_D3 || a.sm_mode == SM_D4);  // twiddles before the first stage
 
   // ---- first stage, its inputs copied to z1 where the lanes read along the
   // line (or the values need their line's exponent, or mirror a half
@@ -352,7 +382,7 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
   t.zo = t.p * pitch;
   const int zc = z1 + t.p * pitch;
   bool direct = false;
-  if constexpr (!XF && OP != OP_C2R) {
+  if constexpr (!XF && OP != OP_C2R && !R2R) {
     direct = lanes && !spectral;
     if (direct) {
       const int64_t off = ioff + (t.p * (packed ? 2 : 1)) * sst;
@@ -364,9 +394,12 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
   }
   if (!direct) {
     MC* zr = reinterpret_cast<MC*>(z) + z1;  // raw values (xf: doubles, converted at the first stage)
-    const int n = OP == OP_C2R ? m : M;
+    const int points = OP == OP_C2R ? m : R2R ? n : M;
     unsigned emx = 0;
-    SmWalk w(lanes, n, a.sm_din, TW, t.p, t.b0, t.k, ioff, ssa, packed ? 2 * sst : sst);
+    if constexpr (R2R) {
+      if (a.sm_mode == SM_X && odd && t.b0 == 0) zr[t.p * pitch] = zr[t.p * pitch + M / 2] = MC{0, 0};
+    }
+    SmWalk w(lanes, points, a.sm_din, TW, t.p, t.b0, t.k, ioff, ssa, packed ? 2 * sst : sst);
     if constexpr (OP == OP_C2R) {
       const MC* in = reinterpret_cast<const MC*>(a.in);
 #pragma unroll 2
@@ -391,7 +424,7 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
 #pragma unroll 1
       for (; w.left > 0; --w.left, w.next()) {
         const MC x = in1k(w.i, w.k, w.off);
-        zr[w.i * pitch + w.k] = x;
+        put(zr + w.i * pitch, w.k, x);
         if constexpr (XF) emx = max(emx, max(dexp_u(x.x), dexp_u(x.y)));
       }
     } else {
@@ -399,18 +432,19 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
 #pragma unroll 1
       while (w.left > 0) {
         MC x[U];
-        int at[U];
+        int at[U], pt[U];
 #pragma unroll
         for (int q = 0; q < U; ++q) {
           const bool ok = w.left > q;
-          at[q] = ok ? w.i * pitch + w.k : -1;
+          at[q] = ok ? w.i * pitch : -1;
+          pt[q] = w.k;
           x[q] = in1(ok ? w.i : nvalid, w.off);
           w.next();
         }
         w.left -= U;
 #pragma unroll
         for (int q = 0; q < U; ++q) {
-          if (at[q] >= 0) zr[at[q]] = x[q];
+          if (at[q] >= 0) put(zr + at[q], pt[q], x[q]);
           if constexpr (XF) emx = max(emx, max(dexp_u(x[q].x), dexp_u(x[q].y)));
         }
       }
@@ -420,7 +454,8 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
         __syncthreads();
         emx = 0;
         const MC* zl = zr + t.p * pitch;
-        for (int q = t.b0; q < (OP == OP_C2R ? 2 * m : M); q += t.k) {
+        const int held = OP == OP_C2R ? 2 * m : R2R && a.sm_mode == SM_D4 ? n : M;
+        for (int q = t.b0; q < held; q += t.k) {
           const MC x = zl[q];
           emx = max(emx, max(dexp_u(x.x), dexp_u(x.y)));
         }
@@ -428,6 +463,38 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
       atomicMax(&lm[0][t.p], emx);
     }
     __syncthreads();
+    if constexpr (R2R) {
+      if (pre) {  // in place: a thread holds both points of each pair
+        const MC* zl = reinterpret_cast<const MC*>(z) + zc;
+        const int emax = XF ? (int)lm[0][t.p] : 0;
+        const float fs = XF ? xf_frac_scale(emax) : 0.0f;
+        auto val = [&](MC x) {
+          if constexpr (XF) return mk(d2xf(x.x, emax, fs, bits), d2xf(x.y, emax, fs, bits));
+          else return mk(x.x, x.y);
+        };
+        if (a.sm_mode == SM_D3) {  // conj(w_k) (x[k] - i x[n - k])
+          for (int k = t.b0; 2 * k <= n; k += t.k) {
+            const Cx<R> A = val(zl[k]);
+            if (k == 0) {
+              if constexpr (XF) z[zc] = mk(xf_shift(A.re, 1), xf_shift(A.im, 1));
+              else z[zc] = A;
+            } else {
+              const Cx<R> B = val(zl[n - k]);
+              z[zc + k] = tw_mul<R, 1>(A + mul_mi(B), a.d23_tab, k);
+              if (2 * k != n) z[zc + n - k] = tw_mul<R, 1>(B + mul_mi(A), a.d23_tab, n - k);
+            }
+          }
+        } else {
+          for (int j = t.b0; j < n; j += t.k) {
+            const Cx<R> A = val(zl[j]);
+            const Cx<R> B = tw_mul<R, -1>(A, a.d23_tab, 2 * n - 1 - j);
+            z[zc + j] = tw_mul<R, -1>(A, a.d23_tab, j);
+            z[zc + 2 * n - 1 - j] = odd ? B : -B;
+          }
+        }
+        __syncthreads();
+      }
+    }
     if constexpr (XF) {
       const int emax = (int)lm[0][t.p];
       const float fs = xf_frac_scale(emax);
@@ -437,14 +504,15 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
         if constexpr (OP == OP_C2R) {
           const int k = pos < m ? pos : M - pos;
           const MC qa = zl[k], qb = zl[m + k];
-          Cx<R> A = mk(d2xf<BITS>(qa.x, emax, fs), d2xf<BITS>(qa.y, emax, fs));
-          Cx<R> B = mk(d2xf<BITS>(qb.x, emax, fs), d2xf<BITS>(qb.y, emax, fs));
+          Cx<R> A = mk(d2xf(qa.x, emax, fs, bits), d2xf(qa.y, emax, fs, bits));
+          Cx<R> B = mk(d2xf(qb.x, emax, fs, bits), d2xf(qb.y, emax, fs, bits));
           if (k == 0 || 2 * k == M) { A.im = xf(0, 0.0f); B.im = xf(0, 0.0f); }
           if (pos >= m) { A.im = -A.im; B.im = -B.im; }
           return mk(A.re - B.im, A.im + B.re);
         } else {
+          if (R2R && pre) return z[zc + pos];
           const MC x = zl[pos];
-          return mk(d2xf<BITS>(x.x, emax, fs), d2xf<BITS>(x.y, emax, fs));
+          return mk(d2xf(x.x, emax, fs, bits), d2xf(x.y, emax, fs, bits));
         }
       });
     } else {
@@ -453,7 +521,7 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
   }
 
   // ---- the other stages ----
-  int Ls = a.sm_r[0], shifts = 0;
+  int Ls = a.sm_r[0], shifts = pre ? 1 : 0;
   int za = 0, zb = z1;  // output of the last stage, the other buffer
 #pragma unroll 1
   for (int s = 1; s < a.sm_nst; ++s) {
@@ -461,7 +529,7 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
     __syncthreads();
     if constexpr (XF) {
       const int r = a.sm_r[s];
-      t.sh = xf_stage_shift(lm[s][t.p], (r <= 2 ? 1 : r <= 4 ? 2 : 3) + HEAD);
+      t.sh = xf_stage_shift(lm[s][t.p], (r <= 2 ? 1 : r <= 4 ? 2 : 3) + head);
       shifts += t.sh;
     }
     t.zi = za + t.p * pitch;
@@ -472,9 +540,10 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
     za = zb;
     zb = x;
   }
+  if constexpr (XF && R2R) shifts += a.sm_mode == SM_D2 || a.sm_mode == SM_D4 ? 1 : 0;  // twiddles after the last
   if constexpr (XF) {
     // the unit's exponent with the line's (r2c: its factor 1/2), and the normalisation's
-    if (t.b0 == 0) loff[t.p] = 127 - BITS + shifts + (int)lm[0][t.p] + a.emax_shift - 254 + a.scale_xe - (OP == OP_R2C ? 1 : 0);
+    if (t.b0 == 0) loff[t.p] = 127 - bits + shifts + (int)lm[0][t.p] + a.emax_shift - 254 + a.scale_xe - (OP == OP_R2C ? 1 : 0);
   }
   __syncthreads();
 
@@ -490,15 +559,30 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
     }
     return q;
   };
-  SmWalk w(a.out_tfast != 0, OP == OP_R2C ? m : M, a.sm_dout, TW, t.p, t.b0, t.k, o.ooff, a.out_sa,
+  // output k of an R2R line
+  auto post = [&](const Cx<R>* zl, int k) {
+    if (a.sm_mode == SM_D2) {
+      const int q = odd == 1 ? n - 1 - k : k;
+      const Cx<R> V = zl[q], W = zl[q == 0 ? 0 : n - q], S = V + W, D = V - W;
+      return mk(tw_mul<R, -1>(mk(S.re, D.im), a.d23_tab, q).re, tw_mul<R, -1>(mk(S.im, -D.re), a.d23_tab, q).re);
+    }
+    if (a.sm_mode == SM_D3) {  // the DFT of the other sign: outputs backwards
+      const int q = even_odd(k);
+      const Cx<R> y = zl[q == 0 ? 0 : n - q];
+      return odd && (k & 1) ? -y : y;
+    }
+    const Cx<R> y = a.sm_mode == SM_X ? zl[k + (odd ? 1 : 0)] : tw_mul<R, -1>(zl[k], a.d23_tab, 2 * n + k);
+    return odd ? mul_i(y) : y;
+  };
+  SmWalk w(a.out_tfast != 0, OP == OP_R2C ? m : R2R ? n : M, a.sm_dout, TW, t.p, t.b0, t.k, o.ooff, a.out_sa,
            packed ? 2 * a.out_st : a.out_st);
 #pragma unroll 2
   for (; w.left > 0; --w.left, w.next()) {
     const int i = w.i, k = w.k;
     const Cx<R>* zl = z + za + i * pitch;
-    if constexpr (OP == OP_C2C) {
+    if constexpr (CIN) {
       if (i >= nvalid) continue;
-      MC y = out1(zl[k], i);
+      MC y = out1(R2R ? post(zl, k) : zl[k], i);
       if (a.deriv == 2) {  // fused spectral derivative on the output
         const int64_t idx = a.deriv_role == 0 ? (int64_t)k : a.deriv_role == 1 ? o.t0 + i : o.didx;
         if constexpr (XF) {
@@ -520,8 +604,8 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
       MC* out = reinterpret_cast<MC*>(a.out) + w.off;
       if (2 * i < nvalid) out[0] = out1(A, i);
       if (2 * i + 1 < nvalid) out[a.out_st] = out1(B, i);
-    } else {  // C2R: real outputs of lines 2 i and 2 i + 1
-      const MC y = out1(zl[k], i);
+    } else {  // real outputs of lines 2 i and 2 i + 1
+      const MC y = out1(R2R ? post(zl, k) : zl[k], i);
       MR* out = reinterpret_cast<MR*>(a.out) + w.off;
       if (2 * i < nvalid) out[0] = y.x;
       if (2 * i + 1 < nvalid) out[a.out_st] = y.y;

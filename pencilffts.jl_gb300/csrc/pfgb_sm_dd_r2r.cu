@@ -1,0 +1,13 @@
+// Smooth-length pass, integer-float pairs for Float64 data, R2R lines (complex, or two real lines as one).
+#include <cuda_runtime.h>
+
+#include "pencilfft_gb300.h"
+#include "pfgb_sm.cuh"
+
+namespace pfgb {
+
+int launch_sm_dd_r2r(bool cplx, const FastArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s) {
+  return cplx ? launch_sm_one<xf, -1, OP_R2R_C>(A, grid, threads, smem, s) : launch_sm_one<xf, -1, OP_R2R_R>(A, grid, threads, smem, s);
+}
+
+}  // namespace pfgb

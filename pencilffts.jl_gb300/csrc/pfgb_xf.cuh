@@ -191,7 +191,7 @@ __device__ __forceinline__ dd xf2dd(xf a, unsigned ue) {
   return dd(f_mul(hi, g), f_mul(lo, g));
 }
 
-// x as a count of 2^(emax - 1023 - B) (B <= 26 bits; emax: the line's largest
+// x as a count of 2^(emax - 1023 - B) (20 < B <= 27 bits; emax: the line's largest
 // biased exponent), fs = xf_frac_scale(emax): the 53-bit significand shifted
 // right in 64 bits, its low word as the fraction.  Zeros and subnormals give
 // zero; a line with a NaN or an infinity gets NaN fractions.  No branch, where
@@ -199,8 +199,7 @@ __device__ __forceinline__ dd xf2dd(xf a, unsigned ue) {
 __device__ __forceinline__ float xf_frac_scale(int emax) {
   return __uint_as_float(emax >= 0x7FF ? 0x7FC00000u : 0x2F800000u);  // 2^-32
 }
-template <int B>
-__device__ __forceinline__ xf d2xf(double x, int emax, float fs) {
+__device__ __forceinline__ xf d2xf(double x, int emax, float fs, int B) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const unsigned hi32 = (unsigned)(b >> 32), lo32 = (unsigned)b;
   const int e = (int)((hi32 >> 20) & 0x7FF);
@@ -210,6 +209,10 @@ __device__ __forceinline__ xf d2xf(double x, int emax, float fs) {
   const int s = (int)hi32 >> 31;
   const float l = __uint2float_rn((unsigned)f) * __uint_as_float(__float_as_uint(fs) | (hi32 & 0x80000000u));
   return xf(((int)(f >> 32) ^ s) - s, l);
+}
+template <int B>
+__device__ __forceinline__ xf d2xf(double x, int emax, float fs) {
+  return d2xf(x, emax, fs, B);
 }
 
 // A rare result of xf2d: zero, NaN (a NaN or infinite fraction, overflow).

@@ -30,7 +30,8 @@ SOURCES = ["pfgb_persist.cu", "pfgb_plan.cu", "pfgb_kernels.cu", "pfgb_noalloc.c
     f"pfgb_fast_dd_d23c_{iom}.cu" for iom in (0, 1, 2, 3)] + ["pfgb_fast_dd_d23r_0.cu"] + [
     f"pfgb_fast_dd_csum_{iom}.cu" for iom in (0, 2)] + ["pfgb_fast_dd_c2ct_0.cu"] + [
     f"pfgb_mr_{t}_{op}_{r0}.cu" for t in ("f32", "dd") for op in ("c2c", "r2c", "c2r") for r0 in (3, 5)] + [
-    f"pfgb_{k}_{t}_{op}.cu" for k in ("bs", "sm") for t in ("f32", "dd") for op in ("c2c", "r2c", "c2r")]
+    f"pfgb_{k}_{t}_{op}.cu" for k in ("bs", "sm") for t in ("f32", "dd") for op in ("c2c", "r2c", "c2r")] + [
+    f"pfgb_sm_{t}_r2r.cu" for t in ("f32", "dd")]
 
 
 def _nvcc():

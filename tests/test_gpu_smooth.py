@@ -120,3 +120,43 @@ def test_sm_in_place_and_batch(cuda):
         for p, x, v, w in keep:
             assert rel(v.to_logical(), oracle_plan(p).forward(x)) <= 2e-6
             assert rel(w.to_logical(), x) <= 2e-6
+
+
+# D2 / D3 (odd and even n), X and D4 lines: DFTs of 6 points to the longest of
+# each type, odd extensions' zeros, one and several stages
+@pytest.mark.parametrize("real", [F64, F32])
+@pytest.mark.parametrize("kind,sizes", [(T.REDFT10, (6, 9, 25, 60, 100, 343, 1000)),
+                                        (T.RODFT10, (6, 7, 63, 96, 500)),
+                                        (T.REDFT01, (7, 10, 45, 120, 960)),
+                                        (T.RODFT01, (6, 15, 50, 243)),
+                                        (T.DHT, (6, 12, 35, 200, 2025)),
+                                        (T.REDFT00, (4, 46, 97, 501, 1001)),
+                                        (T.RODFT00, (2, 5, 44, 299, 999)),
+                                        (T.REDFT11, (3, 5, 50, 105, 1000)),
+                                        (T.RODFT11, (3, 6, 75, 1000))])
+def test_sm_r2r_lines(cuda, real, kind, sizes):
+    r = T.R2R(kind)
+    for n in sizes + ((3000,) if real == F32 and kind in (T.REDFT10, T.RODFT01) else ()):
+        for dims, trs in (((n, 19), (r, T.NoTransform())), ((18, n, 2), (T.NoTransform(), r, T.NoTransform())),
+                          ((9, n), (T.FFT(), r)), ((n, 10), (r, T.FFT()))):
+            plan = P.PencilFFTPlan(dims, trs, real, permute_dims=n % 2 == 0)
+            check_plan(plan, seed=n)
+            assert "sm_pass" in kernels(plan)
+
+
+def test_sm_r2r_spectral_operator(cuda):
+    """A derivative along a Fourier dimension, fused into the R2R pass at the
+    plan's end (Float64), on its output and on its input."""
+    plan = P.PencilFFTPlan((20, 18, 25), (T.RFFT(), T.FFT(), T.R2R(T.REDFT10)), F64)
+    orc = oracle_plan(plan)
+    x = random_input(plan, 3)
+    spec = orc.forward(x)
+    S = plan.allocate_output()
+    S.copy_from_logical(spec)
+    for d, L in ((0, 2 * np.pi), (1, 3.0)):
+        A, B = plan.allocate_input(), plan.allocate_output()
+        A.copy_from_logical(x)
+        P.mul_(B, plan, A, deriv=(d + 1, L))
+        assert rel(B.to_logical(), O.wavenumbers(orc, d, L) * spec) <= 1e-13
+        P.ldiv_(A, plan, S, deriv=(d + 1, L))
+        assert rel(A.to_logical(), orc.ldiv(O.wavenumbers(orc, d, L) * spec)) <= 1e-13

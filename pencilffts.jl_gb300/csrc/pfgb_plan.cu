@@ -127,7 +127,7 @@ struct Pass {
   // smooth-length pass (sm_pass): radices, butterfly step of a thread
   bool sm = false;
   int sm_mode = 0;  // R2R lines (SmMode)
-  int sm_nst = 0, sm_r[kSmStages] = {};
+  int sm_nst = 0, sm_r[kSmStages] = {}, sm_pitch = 0;
   // Bluestein register pass (bs_pass) for other lines up to 2048 points:
   // convolution length 2^logl (ftw holds its twiddles), chirp and filter
   // tables; the generic kernel's geometry is kept (g_*) for executions it
@@ -786,20 +786,48 @@ static int upload_sm_vec(pfgb_plan* P, const std::string& key, const std::vector
   return PFGB_OK;
 }
 
+// Pitch of a line of M points in the tile's buffers: lanes hold w lines side by
+// side, then the next butterfly, whose inputs (and outputs after the first
+// stage of radix r0) lie one element on.  Of the pitches up to one period of
+// the banks above the shortest, the one with the fewest bank conflicts
+// (Float32: 16 elements a period; odd pitches alone left 10 to 20 of 34
+// wavefronts to conflicts at widths such as 9 or 21).
+static int sm_best_pitch(int M, int w, int q, int r0, int ebytes) {
+  const int period = 128 / ebytes, first = M + 2;
+  int best = first;
+  int64_t least = -1;
+  for (int pitch = first; pitch < first + period; ++pitch) {
+    int64_t cost = 0;
+    for (int t0 = 0; t0 < w * q; t0 += period) {
+      int reads[16] = {}, writes[16] = {}, mr = 0, mw = 0;
+      for (int t = t0; t < std::min(t0 + period, w * q); ++t) {
+        const int at = t % w * pitch, b = t / w;
+        mr = std::max(mr, ++reads[(at + b) % period]);
+        mw = std::max(mw, ++writes[(at + b * r0) % period]);
+      }
+      cost += 4 * mr + mw;
+    }
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = pitch;
+    }
+  }
+  return best;
+}
+
 // The smooth-length form of a c2c / r2c / c2r pass of ps.M points (2, 3, 5 and
 // 7 only): radices, lines of a tile and threads, twiddle tables; taken = false
 // if the pass does not take it.  It takes every length that has no
 // power-of-two form, on Float64 data also those of the mixed-radix pass
 // (3 or 5 times a power of two; its Float32 form stays the faster one: 384^3
-// 0.85 ms, where 360^3 takes 0.93 here), with 16 complex lines or more.  Fewer
+// 0.86 ms, where 360^3 takes 0.83 here), with 16 complex lines or more.  Fewer
 // lines keep the Bluestein or mixed-radix tile where those have the length
 // (few): launch latency sets their time, and the plans that ask for those
 // kernels by name in tests have few lines.  Measured round trips, Bluestein or
-// (*) mixed-radix tile against this one: Float64 RFFT 100^3 0.213 -> 0.088 ms,
-// 240^3 1.98 -> 0.67, 360^3 9.73 -> 2.6, *384^3 3.97 -> 2.79, FFT *96^3 0.286
-// -> 0.100, *24^3 0.139 -> 0.045, 1000^2 0.260 -> 0.133, 3000^2 (generic
-// kernel) 4.27 -> 0.96; Float32 RFFT 360^3 3.45 -> 0.93, 120^3 0.088 -> 0.069,
-// 50x60x70 0.040 -> 0.041, FFT 200^3 0.629 -> 0.298.
+// (*) mixed-radix tile against this one: Float64 RFFT 100^3 0.213 -> 0.082 ms,
+// 240^3 1.98 -> 0.64, 360^3 9.73 -> 2.42, *384^3 3.97 -> 2.65, FFT *96^3 0.286
+// -> 0.100, *24^3 0.139 -> 0.045, 1000^2 0.260 -> 0.124; Float32 RFFT 360^3 3.45 -> 0.83, 120^3 0.088 -> 0.069,
+// 50x60x70 0.040 -> 0.041, FFT 200^3 0.629 -> 0.274.
 //
 // The tile: w lines and a butterfly step q (w q threads), by the share of
 // threads that have work in every stage, the threads in flight on an SM, 64
@@ -819,7 +847,7 @@ static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
     if (d != ps.axis && d != td) outer *= ps.lin.size[d];
   if (ncl * outer < 16 && !few) return PFGB_OK;
   const bool strided = ps.lin.perm[0] != ps.axis || ps.lout.perm[0] != ps.axis;
-  const int pitch = (M + 2) | 1, ebytes = f64 ? 16 : 8;
+  const int ebytes = f64 ? 16 : 8, pitch = M + 1 + 128 / ebytes;  // the widest sm_best_pitch gives
   double best = 1e30;
   int tw = 0, k = 0;
   for (int w = 1; w <= kSmLines && w <= std::max<int64_t>(ncl, 1); ++w) {
@@ -868,7 +896,8 @@ static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
   ps.clines = tw;
   ps.lines = pk ? 2 * tw : tw;
   ps.threads = tw * k;
-  ps.smem = (size_t)2 * tw * pitch * ebytes;
+  ps.sm_pitch = sm_best_pitch(M, tw, k, r[0], ebytes);
+  ps.smem = (size_t)2 * tw * ps.sm_pitch * ebytes;
   taken = true;
   return PFGB_OK;
 }
@@ -1420,7 +1449,7 @@ static int make_fast_args(const pfgb_plan* P, const Pass& ps, const void* in, vo
   if (ps.sm) {
     F.sm_m = ps.M;
     F.sm_tw = ps.clines;
-    F.sm_pitch = (ps.M + 2) | 1;
+    F.sm_pitch = ps.sm_pitch;
     F.sm_nst = ps.sm_nst;
     int Ls = 1, at = 0;
     for (int s = 0; s < ps.sm_nst; ++s) {

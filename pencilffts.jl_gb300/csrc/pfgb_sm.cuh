@@ -6,10 +6,15 @@
 // A tile of TW lines goes through nst Stockham stages of mixed radix between
 // two shared-memory buffers.  A thread owns one line of the tile (p = thread
 // mod TW) and every K-th butterfly of each stage: its loads, twiddles and
-// stores need no division, its line's scale is its own, and with the lines
-// consecutive across a warp an odd pitch makes every shared access free of
-// bank conflicts.  Radices up to 16 (Float32) or 8 (Float64, whose range bound
+// stores need no division, its line's scale is its own, and the pitch leaves the
+// fewest bank conflicts for the tile's width (sm_best_pitch).  Radices up to 16 (Float32) or 8 (Float64, whose range bound
 // is a growth of 8 per stage) leave two or three stages for most lengths.
+//
+// Bound by issue slots (125 to 155 instructions a point in Float32, half of
+// them integer, before addresses were stepped in bytes) and the shared-memory
+// pipe together: 360^3 Float32 round trip 930 -> 834 us, Float64 2514 -> 2421 us
+// with byte steps, walks of their own for lanes across the lines, and the
+// pitch.
 //
 // Against the Bluestein tile, which takes these lengths through two
 // power-of-two transforms of at least twice the length: see sm_form in
@@ -162,37 +167,53 @@ __device__ __forceinline__ Cx<R>* sm_z() {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   return reinterpret_cast<Cx<R>*>(smem_raw);
 }
-// A thread's walk over the n points of each of the tile's lines, at array
-// offset off: along its own line in steps of the butterfly step (lanes side by
-// side on different lines) or along the lines one after the other, as the
-// array's contiguous dimension asks.  One division a tile, none a point.
+// A thread's walk over the points of the tile's lines, at array offset off and
+// element at of the buffer.  ACROSS: along its own line in steps of the
+// butterfly step (lanes side by side on different lines); else along the lines
+// one after the other.  The array's contiguous dimension decides.  One
+// division a tile, none a point.
+template <bool ACROSS>
 struct SmWalk {
-  int i, k, left;      // line, point, points left to this thread
+  int i, k, left, at;  // line, point, points left to this thread
   int64_t off;
-  int di, dk, wrap, n;
+  int di, dk, dat, n, pitch;
   int64_t step, turn;
-  __device__ __forceinline__ SmWalk(bool across, int points, Div31 d, int tw, int p, int b0, int step_b, int64_t base,
+  __device__ __forceinline__ SmWalk(int points, Div31 d, int tw, int pitch_, int p, int b0, int step_b, int64_t base,
                                     int64_t sa, int64_t st) {
     const int nt = blockDim.x, tid = threadIdx.x;
     n = points;
-    i = across ? p : (int)div31((unsigned)tid, d);
-    k = across ? b0 : tid - i * n;
-    left = across ? (n - b0 + step_b - 1) / step_b : (tw * n - tid + nt - 1) / nt;
-    di = across ? 0 : (int)div31((unsigned)nt, d);
-    dk = across ? step_b : nt - di * n;
-    wrap = across ? 0x7FFFFFFF : n;
+    pitch = pitch_;
+    if constexpr (ACROSS) {
+      i = p;
+      k = b0;
+      left = (n - b0 + step_b - 1) / step_b;
+      di = 0;
+      dk = step_b;
+    } else {
+      i = (int)div31((unsigned)tid, d);
+      k = tid - i * n;
+      left = (tw * n - tid + nt - 1) / nt;
+      di = (int)div31((unsigned)nt, d);
+      dk = nt - di * n;
+    }
+    at = i * pitch + k;
+    dat = di * pitch + dk;
     off = base + k * sa + i * st;
     step = dk * sa + di * st;
     turn = st - n * sa;
   }
   __device__ __forceinline__ void next() {
-    i += di;
     k += dk;
+    at += dat;
     off += step;
-    if (k >= wrap) {
-      k -= n;
-      ++i;
-      off += turn;
+    if constexpr (!ACROSS) {
+      i += di;
+      if (k >= n) {
+        k -= n;
+        at += pitch - n;
+        ++i;
+        off += turn;
+      }
     }
   }
 };
@@ -215,6 +236,11 @@ __device__ __forceinline__ void sm_stage(const FastArgs& a, int s, SmThread& t, 
   const void* tw = a.tw;
   if constexpr (XF) tw = reinterpret_cast<const int4*>(a.tw) + (t.sh - 1) * a.sm_ntw;
   int hi = 0, lo = 0;
+  // byte steps between a butterfly's inputs, outputs and twiddles (one
+  // multiply-add an access: a third of the instructions were addresses)
+  constexpr unsigned EB = sizeof(Cx<R>);
+  const unsigned dT = T * EB, dL = Ls * EB;
+#pragma unroll 1
   for (int b = t.b0; b < T; b += t.k) {
     Cx<R> v[RAD];
     int j = 0;
@@ -223,17 +249,18 @@ __device__ __forceinline__ void sm_stage(const FastArgs& a, int s, SmThread& t, 
       for (int q = 0; q < RAD; ++q) v[q] = ld(b, q, T);
     } else {
       j = b - (int)div31((unsigned)b, a.sm_ls[s]) * Ls;
-      const int e0 = a.sm_tw0[s] + j;
+      const char* zr = reinterpret_cast<const char*>(z + t.zi + b);
+      const char* tp = reinterpret_cast<const char*>(tw) + (size_t)(unsigned)(a.sm_tw0[s] + j) * EB;
 #pragma unroll
-      for (int q = 0; q < RAD; ++q) v[q] = z[t.zi + b + q * T];
+      for (int q = 0; q < RAD; ++q) v[q] = *reinterpret_cast<const Cx<R>*>(zr + q * dT);
 #pragma unroll
-      for (int q = 1; q < RAD; ++q) v[q] = tw_mul<R, SIGN>(v[q], tw, e0 + (q - 1) * Ls);
+      for (int q = 1; q < RAD; ++q) v[q] = tw_mul<R, SIGN>(v[q], tp + (size_t)(q - 1) * dL, 0);
       if constexpr (XF) v[0] = mk(xf_shift(v[0].re, t.sh), xf_shift(v[0].im, t.sh));
     }
     sm_dft<RAD, SIGN>(v);
-    const int zw = t.zo + (b - j) * RAD + j;
+    char* zw = reinterpret_cast<char*>(z + t.zo + (b - j) * RAD + j);
 #pragma unroll
-    for (int q = 0; q < RAD; ++q) z[zw + q * Ls] = v[q];
+    for (int q = 0; q < RAD; ++q) *reinterpret_cast<Cx<R>*>(zw + q * dL) = v[q];
     if constexpr (XF) {
 #pragma unroll
       for (int q = 0; q < RAD; ++q) {
@@ -399,56 +426,59 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
     if constexpr (R2R) {
       if (a.sm_mode == SM_X && odd && t.b0 == 0) zr[t.p * pitch] = zr[t.p * pitch + M / 2] = MC{0, 0};
     }
-    SmWalk w(lanes, points, a.sm_din, TW, t.p, t.b0, t.k, ioff, ssa, packed ? 2 * sst : sst);
-    if constexpr (OP == OP_C2R) {
-      const MC* in = reinterpret_cast<const MC*>(a.in);
+    auto load = [&](auto w) {
+      if constexpr (OP == OP_C2R) {
+        const MC* in = reinterpret_cast<const MC*>(a.in);
 #pragma unroll 2
-      for (; w.left > 0; --w.left, w.next()) {
-        const int k = w.k;
-        MC A{0, 0}, B{0, 0};
-        if (2 * w.i < nvalid) A = in[w.off];
-        if (2 * w.i + 1 < nvalid) B = in[w.off + sst];
-        MC* zl = zr + w.i * pitch;
-        if constexpr (XF) {
-          zl[k] = A;
-          zl[m + k] = B;
-          emx = max(emx, max(max(dexp_u(A.x), dexp_u(A.y)), max(dexp_u(B.x), dexp_u(B.y))));
-        } else if (k == 0 || 2 * k == M) {
-          zl[k] = MC{A.x, B.x};
-        } else {  // A + i B, and conj(A) + i conj(B) at M - k
-          zl[k] = MC{A.x - B.y, A.y + B.x};
-          zl[M - k] = MC{A.x + B.y, B.x - A.y};
+        for (; w.left > 0; --w.left, w.next()) {
+          const int k = w.k;
+          MC A{0, 0}, B{0, 0};
+          if (2 * w.i < nvalid) A = in[w.off];
+          if (2 * w.i + 1 < nvalid) B = in[w.off + sst];
+          MC* zk = zr + w.at;
+          if constexpr (XF) {
+            zk[0] = A;
+            zk[m] = B;
+            emx = max(emx, max(max(dexp_u(A.x), dexp_u(A.y)), max(dexp_u(B.x), dexp_u(B.y))));
+          } else if (k == 0 || 2 * k == M) {
+            zk[0] = MC{A.x, B.x};
+          } else {  // A + i B, and conj(A) + i conj(B) at M - k
+            zk[0] = MC{A.x - B.y, A.y + B.x};
+            zk[M - 2 * k] = MC{A.x + B.y, B.x - A.y};
+          }
         }
-      }
-    } else if (spectral) {
+      } else if (spectral) {
 #pragma unroll 1
-      for (; w.left > 0; --w.left, w.next()) {
-        const MC x = in1k(w.i, w.k, w.off);
-        put(zr + w.i * pitch, w.k, x);
-        if constexpr (XF) emx = max(emx, max(dexp_u(x.x), dexp_u(x.y)));
-      }
-    } else {
-      constexpr int U = XF ? 4 : 8;  // loads in flight a thread
+        for (; w.left > 0; --w.left, w.next()) {
+          const MC x = in1k(w.i, w.k, w.off);
+          put(zr + w.at - w.k, w.k, x);
+          if constexpr (XF) emx = max(emx, max(dexp_u(x.x), dexp_u(x.y)));
+        }
+      } else {
+        constexpr int U = XF ? 4 : 8;  // loads in flight a thread
 #pragma unroll 1
-      while (w.left > 0) {
-        MC x[U];
-        int at[U], pt[U];
+        while (w.left > 0) {
+          MC x[U];
+          int at[U], pt[U];
 #pragma unroll
-        for (int q = 0; q < U; ++q) {
-          const bool ok = w.left > q;
-          at[q] = ok ? w.i * pitch : -1;
-          pt[q] = w.k;
-          x[q] = in1(ok ? w.i : nvalid, w.off);
-          w.next();
-        }
-        w.left -= U;
+          for (int q = 0; q < U; ++q) {
+            const bool ok = w.left > q;
+            at[q] = ok ? w.at : -1;
+            pt[q] = w.k;
+            x[q] = in1(ok ? w.i : nvalid, w.off);
+            w.next();
+          }
+          w.left -= U;
 #pragma unroll
-        for (int q = 0; q < U; ++q) {
-          if (at[q] >= 0) put(zr + at[q], pt[q], x[q]);
-          if constexpr (XF) emx = max(emx, max(dexp_u(x[q].x), dexp_u(x[q].y)));
+          for (int q = 0; q < U; ++q) {
+            if (at[q] >= 0) put(zr + at[q] - pt[q], pt[q], x[q]);
+            if constexpr (XF) emx = max(emx, max(dexp_u(x[q].x), dexp_u(x[q].y)));
+          }
         }
       }
-    }
+    };
+    if (lanes) load(SmWalk<true>(points, a.sm_din, TW, pitch, t.p, t.b0, t.k, ioff, ssa, packed ? 2 * sst : sst));
+    else load(SmWalk<false>(points, a.sm_din, TW, pitch, t.p, t.b0, t.k, ioff, ssa, packed ? 2 * sst : sst));
     if constexpr (XF) {
       if (!lanes) {  // lines along the lanes: each line's own threads look it over
         __syncthreads();
@@ -574,43 +604,47 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
     const Cx<R> y = a.sm_mode == SM_X ? zl[k + (odd ? 1 : 0)] : tw_mul<R, -1>(zl[k], a.d23_tab, 2 * n + k);
     return odd ? mul_i(y) : y;
   };
-  SmWalk w(a.out_tfast != 0, OP == OP_R2C ? m : R2R ? n : M, a.sm_dout, TW, t.p, t.b0, t.k, o.ooff, a.out_sa,
-           packed ? 2 * a.out_st : a.out_st);
+  auto store = [&](auto w) {
 #pragma unroll 2
-  for (; w.left > 0; --w.left, w.next()) {
-    const int i = w.i, k = w.k;
-    const Cx<R>* zl = z + za + i * pitch;
-    if constexpr (CIN) {
-      if (i >= nvalid) continue;
-      MC y = out1(R2R ? post(zl, k) : zl[k], i);
-      if (a.deriv == 2) {  // fused spectral derivative on the output
-        const int64_t idx = a.deriv_role == 0 ? (int64_t)k : a.deriv_role == 1 ? o.t0 + i : o.didx;
-        if constexpr (XF) {
-          const double kk = sm_k(idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
-          y = MC{-y.y * kk, y.x * kk};
-        } else {
-          const Cx<float> q = mul_ik(mk(y.x, y.y), idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
-          y = MC{q.re, q.im};
+    for (; w.left > 0; --w.left, w.next()) {
+      const int i = w.i, k = w.k;
+      const Cx<R>* zl = z + za + w.at - k;
+      if constexpr (CIN) {
+        if (i >= nvalid) continue;
+        MC y = out1(R2R ? post(zl, k) : zl[k], i);
+        if (a.deriv == 2) {  // fused spectral derivative on the output
+          const int64_t idx = a.deriv_role == 0 ? (int64_t)k : a.deriv_role == 1 ? o.t0 + i : o.didx;
+          if constexpr (XF) {
+            const double kk = sm_k(idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
+            y = MC{-y.y * kk, y.x * kk};
+          } else {
+            const Cx<float> q = mul_ik(mk(y.x, y.y), idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
+            y = MC{q.re, q.im};
+          }
         }
+        reinterpret_cast<MC*>(a.out)[w.off] = y;
+      } else if constexpr (OP == OP_R2C) {
+        const Cx<R> f = zl[k], g = conj(zl[k == 0 ? 0 : M - k]);
+        Cx<R> A = f + g, B = mul_mi(f - g);
+        if constexpr (!XF) {
+          A = mk(half(A.re), half(A.im));
+          B = mk(half(B.re), half(B.im));
+        }
+        MC* out = reinterpret_cast<MC*>(a.out) + w.off;
+        if (2 * i < nvalid) out[0] = out1(A, i);
+        if (2 * i + 1 < nvalid) out[a.out_st] = out1(B, i);
+      } else {  // real outputs of lines 2 i and 2 i + 1
+        const MC y = out1(R2R ? post(zl, k) : zl[k], i);
+        MR* out = reinterpret_cast<MR*>(a.out) + w.off;
+        if (2 * i < nvalid) out[0] = y.x;
+        if (2 * i + 1 < nvalid) out[a.out_st] = y.y;
       }
-      reinterpret_cast<MC*>(a.out)[w.off] = y;
-    } else if constexpr (OP == OP_R2C) {
-      const Cx<R> f = zl[k], g = conj(zl[k == 0 ? 0 : M - k]);
-      Cx<R> A = f + g, B = mul_mi(f - g);
-      if constexpr (!XF) {
-        A = mk(half(A.re), half(A.im));
-        B = mk(half(B.re), half(B.im));
-      }
-      MC* out = reinterpret_cast<MC*>(a.out) + w.off;
-      if (2 * i < nvalid) out[0] = out1(A, i);
-      if (2 * i + 1 < nvalid) out[a.out_st] = out1(B, i);
-    } else {  // real outputs of lines 2 i and 2 i + 1
-      const MC y = out1(R2R ? post(zl, k) : zl[k], i);
-      MR* out = reinterpret_cast<MR*>(a.out) + w.off;
-      if (2 * i < nvalid) out[0] = y.x;
-      if (2 * i + 1 < nvalid) out[a.out_st] = y.y;
     }
-  }
+  };
+  const int outs = OP == OP_R2C ? m : R2R ? n : M;
+  const int64_t ost = packed ? 2 * a.out_st : a.out_st;
+  if (a.out_tfast) store(SmWalk<true>(outs, a.sm_dout, TW, pitch, t.p, t.b0, t.k, o.ooff, a.out_sa, ost));
+  else store(SmWalk<false>(outs, a.sm_dout, TW, pitch, t.p, t.b0, t.k, o.ooff, a.out_sa, ost));
 }
 
 int fail_cuda(cudaError_t e, const char* what);

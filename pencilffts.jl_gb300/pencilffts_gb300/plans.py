@@ -424,9 +424,12 @@ class PencilFFTPlan:
     # -- execution ---------------------------------------------------------
     def _stream_ptr(self):
         if self._stream is not None:
-            return ctypes.c_void_p(int(self._stream))
+            return int(self._stream)
         torch = _torch()
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        if not torch.cuda.is_initialized():
+            return torch.cuda.current_stream().cuda_stream
+        # the handle alone, without a Stream object (2.9 us of each call)
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
     def _check_arrays(self, A_in, A_out):
         """reference operations.jl:87-127.  ``A_in`` holds data of the plan's
@@ -466,20 +469,16 @@ class PencilFFTPlan:
         if forward:
             self._check_arrays(src, dst)
             if d is None:
-                rc = L.pfgb_forward(self._handle, ctypes.c_void_p(dst.data_ptr()),
-                                    ctypes.c_void_p(src.data_ptr()), stream)
+                rc = L.pfgb_forward(self._handle, dst.data_ptr(), src.data_ptr(), stream)
             else:
-                rc = L.pfgb_forward_deriv(self._handle, ctypes.c_void_p(dst.data_ptr()),
-                                          ctypes.c_void_p(src.data_ptr()), stream, d, s)
+                rc = L.pfgb_forward_deriv(self._handle, dst.data_ptr(), src.data_ptr(), stream, d, s)
             _lib.check(rc, "pfgb_forward")
         else:
             self._check_arrays(dst, src)
             if d is None:
-                rc = L.pfgb_backward(self._handle, ctypes.c_void_p(dst.data_ptr()),
-                                     ctypes.c_void_p(src.data_ptr()), stream, 1 if normalise else 0)
+                rc = L.pfgb_backward(self._handle, dst.data_ptr(), src.data_ptr(), stream, 1 if normalise else 0)
             else:
-                rc = L.pfgb_backward_deriv(self._handle, ctypes.c_void_p(dst.data_ptr()),
-                                           ctypes.c_void_p(src.data_ptr()), stream,
+                rc = L.pfgb_backward_deriv(self._handle, dst.data_ptr(), src.data_ptr(), stream,
                                            1 if normalise else 0, d, s)
             _lib.check(rc, "pfgb_backward")
         return dst

@@ -211,6 +211,7 @@ __host__ __device__ constexpr int bs_min_blocks(int logl) {
 }
 template <typename R, int LOGL, int OP>
 __global__ void __launch_bounds__(bs_threads<R>(LOGL), bs_min_blocks<R>(LOGL)) bs_pass(const FastArgs a) {
+  pass_enter();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   bs_tile<R, LOGL, OP>(a, blockIdx.x, reinterpret_cast<Cx<R>*>(smem_raw));
 }
@@ -224,8 +225,7 @@ static int launch_bs_one(const FastArgs& A, int64_t grid, cudaStream_t s) {
   const size_t smem = bs_smem<R>(LOGL);
   int rc = ensure_smem_attr(bs_pass<R, LOGL, OP>, (int)smem, configured, "cudaFuncSetAttribute(bs_pass)");
   if (rc || grid == 0) return rc;
-  bs_pass<R, LOGL, OP><<<(unsigned)grid, bs_threads<R>(LOGL), smem, s>>>(A);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pass_kernel(bs_pass<R, LOGL, OP>, grid, bs_threads<R>(LOGL), smem, s, A);
   if (e != cudaSuccess) return fail_cuda(e, "bs_pass launch");
   return PFGB_OK;
 }

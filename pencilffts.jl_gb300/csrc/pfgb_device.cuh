@@ -16,6 +16,7 @@
 
 #include "pencilfft_gb300.h"
 #include "pfgb_div31.h"
+#include "pfgb_launch.h"
 
 namespace pfgb {
 
@@ -494,6 +495,7 @@ __device__ __forceinline__ Cx<R> r2r_post(const Cx<R>* zl, const PassArgs& a, in
 // ---------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(1024) pass_kernel(const PassArgs a) {
+  pass_enter();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   Cx<R>* z = reinterpret_cast<Cx<R>*>(smem_raw);
   const int nth = blockDim.x;
@@ -736,6 +738,7 @@ struct LPackArgs {
 
 template <typename E>
 __global__ void copy_kernel(const CopyArgs a) {
+  pass_enter();
   const E* in = reinterpret_cast<const E*>(a.in);
   E* out = reinterpret_cast<E*>(a.out);
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.total;

@@ -749,7 +749,7 @@ __device__ __forceinline__ float pow2_le0(int d) {
   return d >= -126 ? __uint_as_float((unsigned)(d + 127) << 23) : 0.0f;
 }
 __device__ __forceinline__ float te_factor(const FastArgs& a, unsigned tebase, int64_t line, int pos, int erun) {
-  return pow2_le0(__ldg(a.te + te_index(a, tebase, line, pos)) - erun);
+  return pow2_le0(a.te[te_index(a, tebase, line, pos)] - erun);
 }
 template <typename R>
 __device__ __forceinline__ Cx<R> scale_pow2(Cx<R> y, float f) {
@@ -846,7 +846,7 @@ __device__ __forceinline__ void fast_tile_load(const FastArgs& a, int64_t bid, c
         const unsigned te0 = te_index(a, o.tebase, t0 + p, b), dte = ((unsigned)T >> a.te_sh[0]) * a.te_mul[0];
 #pragma unroll
         for (int r = 0; r < P; ++r)
-          tev[r] = p < nvalid ? __ldg(a.te + (T > 1 ? te0 + r * dte : te_index(a, o.tebase, t0 + p, r))) : emax;
+          tev[r] = p < nvalid ? a.te[T > 1 ? te0 + r * dte : te_index(a, o.tebase, t0 + p, r)] : emax;
       }
 #pragma unroll
       for (int r = 0; r < P; ++r) {
@@ -1769,7 +1769,7 @@ __device__ __forceinline__ void fast_tile_fx(const FastArgs& a, int64_t bid, Cx<
       for (int r = 0; r < 8; ++r) {
         const bool ok = p < nvalid;
         q[r] = ok ? in[(int64_t)(b + r * T) * ssa] : make_longlong2(0, 0);
-        tev[r] = ok ? __ldg(a.te_in + te_index(a, o.tebase, t0 + p, b + r * T)) : kTeZero;
+        tev[r] = ok ? a.te_in[te_index(a, o.tebase, t0 + p, b + r * T)] : kTeZero;
         tm = max(tm, tev[r]);
       }
       atomicMax(&red[0][p], tm);
@@ -1824,8 +1824,8 @@ __device__ __forceinline__ void fast_tile_fx(const FastArgs& a, int64_t bid, Cx<
       const int pos = b + r * T;
       const int k = pos < m ? pos : M - pos;
       if constexpr (IN_FX) {
-        ta[r] = i0 < nvalid ? __ldg(a.te_in + te_index(a, o.tebase, t0 + i0, k)) : kTeZero;
-        tb[r] = i1 < nvalid ? __ldg(a.te_in + te_index(a, o.tebase, t0 + i1, k)) : kTeZero;
+        ta[r] = i0 < nvalid ? a.te_in[te_index(a, o.tebase, t0 + i0, k)] : kTeZero;
+        tb[r] = i1 < nvalid ? a.te_in[te_index(a, o.tebase, t0 + i1, k)] : kTeZero;
         tm = max(tm, max(ta[r], tb[r]));
       } else {
         const double2* in = reinterpret_cast<const double2*>(src) + ioff;
@@ -2023,6 +2023,7 @@ __device__ __forceinline__ void fast_tile(const FastArgs& a, int64_t bid, Cx<R>*
 template <typename R, int LOGM, int SIGN, int OP, int IOM>
 __global__ void __launch_bounds__(fast_threads<R>(LOGM, OP), fast_min_blocks<R>(LOGM, OP, IOM))
     fast_pass(const FastArgs a) {
+  pass_enter();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   fast_tile<R, LOGM, SIGN, OP, IOM>(a, blockIdx.x, reinterpret_cast<Cx<R>*>(smem_raw), a.in, -1, a.in_sa, a.in_st);
 }

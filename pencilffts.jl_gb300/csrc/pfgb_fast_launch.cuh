@@ -22,8 +22,7 @@ static int launch_fast_one(const FastArgs& A, int64_t grid, cudaStream_t s) {
   const size_t smem = fast_smem<R>(LOGM, OP);
   int rc = ensure_smem_attr(fast_pass<R, LOGM, SIGN, OP, IOM>, (int)smem, configured, "cudaFuncSetAttribute(fast_pass)");
   if (rc || grid == 0) return rc;
-  fast_pass<R, LOGM, SIGN, OP, IOM><<<(unsigned)grid, fast_threads<R>(LOGM, OP), smem, s>>>(A);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pass_kernel(fast_pass<R, LOGM, SIGN, OP, IOM>, grid, fast_threads<R>(LOGM, OP), smem, s, A);
   if (e != cudaSuccess) return fail_cuda(e, "fast_pass launch");
   return PFGB_OK;
 }

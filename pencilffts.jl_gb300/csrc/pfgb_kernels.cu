@@ -16,8 +16,7 @@ static int launch_pass_t(const PassArgs& A, int64_t grid, int threads, size_t sm
   static bool configured[kMaxDevicesConfigured] = {};
   int rc = ensure_smem_attr(pass_kernel<R>, 200 * 1024, configured, "cudaFuncSetAttribute(pass_kernel)");
   if (rc || grid == 0) return rc;
-  pass_kernel<R><<<(unsigned)grid, threads, smem, s>>>(A);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pass_kernel(pass_kernel<R>, grid, threads, smem, s, A);
   if (e != cudaSuccess) return fail_cuda(e, "pass_kernel launch");
   return PFGB_OK;
 }
@@ -32,12 +31,8 @@ int launch_copy(int elt_bytes, const CopyArgs& C, cudaStream_t s) {
   if (C.total == 0) return PFGB_OK;
   int64_t blocks = (C.total + 255) / 256;
   if (blocks > 152 * 32) blocks = 152 * 32;
-  switch (elt_bytes) {
-    case 4: copy_kernel<float><<<(unsigned)blocks, 256, 0, s>>>(C); break;
-    case 8: copy_kernel<double><<<(unsigned)blocks, 256, 0, s>>>(C); break;
-    default: copy_kernel<double2><<<(unsigned)blocks, 256, 0, s>>>(C); break;
-  }
-  cudaError_t e = cudaGetLastError();
+  const auto kernel = elt_bytes == 4 ? copy_kernel<float> : elt_bytes == 8 ? copy_kernel<double> : copy_kernel<double2>;
+  const cudaError_t e = launch_pass_kernel(kernel, blocks, 256, 0, s, C);
   if (e != cudaSuccess) return fail_cuda(e, "copy_kernel launch");
   return PFGB_OK;
 }
@@ -231,6 +226,7 @@ __device__ __forceinline__ void lp_store(const LPackArgs& a, const LPoint<R>& p)
 // descending run when the line axis is the fastest).
 template <typename R, typename C, bool BIG>
 __global__ void __launch_bounds__(256) lpack_kernel(const LPackArgs a) {
+  pass_enter();
   constexpr int U = sizeof(R) == 8 ? 2 : 4;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t e0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e0 < a.total; e0 += U * stride) {
@@ -247,14 +243,9 @@ int launch_lpack(int real_bytes, const LPackArgs& L, cudaStream_t s) {
   int64_t blocks = (L.total + 255) / 256;
   if (blocks > 152 * 16) blocks = 152 * 16;
   const bool big = L.total >= (int64_t{1} << 31);
-  if (real_bytes == 8) {
-    if (big) lpack_kernel<double, double2, true><<<(unsigned)blocks, 256, 0, s>>>(L);
-    else lpack_kernel<double, double2, false><<<(unsigned)blocks, 256, 0, s>>>(L);
-  } else {
-    if (big) lpack_kernel<float, float2, true><<<(unsigned)blocks, 256, 0, s>>>(L);
-    else lpack_kernel<float, float2, false><<<(unsigned)blocks, 256, 0, s>>>(L);
-  }
-  cudaError_t e = cudaGetLastError();
+  const auto kernel = real_bytes == 8 ? (big ? lpack_kernel<double, double2, true> : lpack_kernel<double, double2, false>)
+                                      : (big ? lpack_kernel<float, float2, true> : lpack_kernel<float, float2, false>);
+  const cudaError_t e = launch_pass_kernel(kernel, blocks, 256, 0, s, L);
   if (e != cudaSuccess) return fail_cuda(e, "lpack_kernel launch");
   return PFGB_OK;
 }

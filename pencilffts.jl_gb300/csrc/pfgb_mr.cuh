@@ -291,6 +291,7 @@ __device__ __forceinline__ void mr_tile(const FastArgs& a, int64_t bid, Cx<R>* z
 
 template <typename R, int R0, int LOGN, int SIGN, int OP>
 __global__ void __launch_bounds__(mr_threads<R>(LOGN)) mr_pass(const FastArgs a) {
+  pass_enter();
   extern __shared__ __align__(128) unsigned char smem_raw[];
   mr_tile<R, R0, LOGN, SIGN, OP>(a, blockIdx.x, reinterpret_cast<Cx<R>*>(smem_raw));
 }
@@ -305,8 +306,7 @@ static int launch_mr_one(const FastArgs& A, int64_t grid, cudaStream_t s) {
   const size_t smem = mr_smem<R>(R0, LOGN, OP);
   int rc = ensure_smem_attr(mr_pass<R, R0, LOGN, SIGN, OP>, (int)smem, configured, "cudaFuncSetAttribute(mr_pass)");
   if (rc || grid == 0) return rc;
-  mr_pass<R, R0, LOGN, SIGN, OP><<<(unsigned)grid, mr_threads<R>(LOGN), smem, s>>>(A);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pass_kernel(mr_pass<R, R0, LOGN, SIGN, OP>, grid, mr_threads<R>(LOGN), smem, s, A);
   if (e != cudaSuccess) return fail_cuda(e, "mr_pass launch");
   return PFGB_OK;
 }

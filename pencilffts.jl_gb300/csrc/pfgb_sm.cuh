@@ -304,6 +304,7 @@ __device__ __forceinline__ double sm_k(int64_t idx, int half, int64_t n, float k
 // Float64.
 template <typename R, int SIGN, int OP>
 __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4) sm_pass(const FastArgs a) {
+  pass_enter();
   constexpr bool XF = std::is_same<R, xf>::value;
   using MR = typename std::conditional<XF, double, float>::type;
   using MC = typename std::conditional<XF, double2, float2>::type;
@@ -655,8 +656,7 @@ static int launch_sm_one(const FastArgs& A, int64_t grid, int threads, size_t sm
   static bool configured[kMaxDevicesConfigured] = {};
   int rc = ensure_smem_attr(sm_pass<R, SIGN, OP>, kSmMaxSmem, configured, "cudaFuncSetAttribute(sm_pass)");
   if (rc || grid == 0) return rc;
-  sm_pass<R, SIGN, OP><<<(unsigned)grid, threads, smem, s>>>(A);
-  cudaError_t e = cudaGetLastError();
+  const cudaError_t e = launch_pass_kernel(sm_pass<R, SIGN, OP>, grid, threads, smem, s, A);
   if (e != cudaSuccess) return fail_cuda(e, "sm_pass launch");
   return PFGB_OK;
 }

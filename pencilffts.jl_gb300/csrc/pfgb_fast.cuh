@@ -169,7 +169,10 @@ __device__ __forceinline__ Cx<R> mul_ik(Cx<R> y, int64_t idx, int half, int64_t 
 //          compute phases interleave (two CTAs: 5.87 ms against 6.58 ms with
 //          one 512-thread CTA; three: 5.43 ms against 5.63 ms with two; four:
 //          4.70 ms against 4.91 ms with three; 128-thread CTAs: 5.81 ms);
-//          512 threads when a line needs them (M = 4096).
+//          512 threads when a line needs them (M = 4096), two CTAs/SM: with
+//          one, nothing covered a line's loads and stores (16384x4096 round
+//          trip, the 4096-point passes 480 and 718 -> 363 and 510 us; tiles of
+//          two lines in one 1024-thread CTA: 445 and 535).
 //   float: 512 threads, 3 CTAs/SM (register cap 42): 1.75 ms against 1.84 ms
 //          with 2 CTAs/SM and 1.80 ms with four 256-thread CTAs.
 #ifndef PFGB_FAST_THREADS_F32
@@ -647,7 +650,7 @@ __host__ __device__ constexpr int fast_min_blocks(int logm, int op, int iom) {
                                2048 / fast_threads<R>(logm, op)
                            ? (op == OP_C2R && PFGB_FAST_F32_MINBLOCKS > 3 ? 3 : PFGB_FAST_F32_MINBLOCKS)
                            : 2048 / fast_threads<R>(logm, op)))
-         : fast_threads<R>(logm, op) >= 512 ? 1
+         : fast_threads<R>(logm, op) >= 512 ? 2
          : (fast_d23(op) || fast_d4(op)) ? 3  // two loads a position (D3) or two real lines (D2R / D3R): ~0.2-0.5 KB of spill at 64 registers
          : PFGB_FAST_DD_MINBLOCKS <= 0 ? 512 / fast_threads<R>(logm, op)
          : (op == OP_C2R && !(iom & 1) && PFGB_FAST_DD_MINBLOCKS > 4) ? 4

@@ -386,6 +386,31 @@ static int upload_fast_table(pfgb_plan* P, int M, const void** out) {
   return PFGB_OK;
 }
 
+// A table of twiddles: float (re, im), or xf_tw for Float64 plans, one after the
+// other for the shifts 1 .. shifts.
+static int upload_shifted(pfgb_plan* P, const std::string& key, const std::vector<std::complex<ld>>& w, int shifts) {
+  std::vector<float> h;
+  if (P->rb == 8) {
+    std::vector<xf_tw_parts> parts;
+    parts.reserve(w.size());
+    for (const auto& x : w) parts.push_back(split_twiddle(x));
+    h.reserve(4 * w.size() * shifts);
+    for (int s = 1; s <= shifts; ++s)
+      for (const auto& x : parts) push_xf_twiddle(h, x, s);
+  } else {
+    h.reserve(2 * w.size());
+    for (const auto& x : w) {
+      h.push_back((float)x.real());
+      h.push_back((float)x.imag());
+    }
+  }
+  void* d = nullptr;
+  PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(float), 16)));
+  P->tables[key] = d;
+  PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
+  return PFGB_OK;
+}
+
 // The register stages' twiddles of a line of 2^logm points with 2^lp points a
 // thread (stage_twiddles): float (re, im), or xf_tw for Float64 plans, one table
 // per shift.
@@ -400,24 +425,11 @@ static int upload_stage_table(pfgb_plan* P, int logm, int lp, const void** out) 
     *out = it->second;
     return PFGB_OK;
   }
-  std::vector<float> h;
-  h.reserve((size_t)12 << logm);
   std::vector<std::complex<ld>> w;
   stage_twiddles(logm, lp, [&](int m) { w.push_back(expi_pi(2 * (int64_t)m, (int64_t)1 << logm)); });
-  for (int s = 1; s <= (P->rb == 8 ? kXfShifts : 1); ++s)
-    for (const auto& x : w) {
-      if (P->rb == 8) {
-        push_xf_twiddle(h, x, s);
-      } else {
-        h.push_back((float)x.real());
-        h.push_back((float)x.imag());
-      }
-    }
-  void* d = nullptr;
-  PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(float), 16)));
-  PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
-  P->tables[key] = d;
-  *out = d;
+  int rc = upload_shifted(P, key, w, kXfShifts);
+  if (rc) return rc;
+  *out = P->tables[key];
   return PFGB_OK;
 }
 // of a power-of-two pass (its points a thread) and of the other register
@@ -766,26 +778,6 @@ static bool sm_radices(int M, bool f64, int& nst, int (&r)[kSmStages]) {
   return best_n <= kSmStages;
 }
 
-// A table of the smooth-length pass: float (re, im), or xf_tw for Float64 plans,
-// one after the other for the shifts 1 .. shifts.
-static int upload_sm_vec(pfgb_plan* P, const std::string& key, const std::vector<std::complex<ld>>& w, int shifts) {
-  std::vector<float> h;
-  for (int s = 1; s <= (P->rb == 8 ? shifts : 1); ++s)
-    for (const auto& x : w) {
-      if (P->rb == 8) {
-        push_xf_twiddle(h, x, s);
-      } else {
-        h.push_back((float)x.real());
-        h.push_back((float)x.imag());
-      }
-    }
-  void* d = nullptr;
-  PFGB_CUDA(cudaMalloc(&d, std::max<size_t>(h.size() * sizeof(float), 16)));
-  P->tables[key] = d;
-  PFGB_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(float), cudaMemcpyHostToDevice));
-  return PFGB_OK;
-}
-
 // Pitch of a line of M points in the tile's buffers: lanes hold w lines side by
 // side, then the next butterfly, whose inputs (and outputs after the first
 // stage of radix r0) lie one element on.  Of the pitches up to one period of
@@ -883,7 +875,7 @@ static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
     for (int s = 1, Ls = r[0]; s < nst; Ls *= r[s], ++s)
       for (int q = 1; q < r[s]; ++q)
         for (int j = 0; j < Ls; ++j) w.push_back(expi_pi(2 * (int64_t)q * j, (int64_t)r[s] * Ls));
-    const int rc = upload_sm_vec(P, key, w, kXfShifts);
+    const int rc = upload_shifted(P, key, w, kXfShifts);
     if (rc) return rc;
   }
   ps.ftw = P->query_only ? nullptr : P->tables[key];
@@ -946,7 +938,7 @@ static int sm_r2r_form(pfgb_plan* P, Pass& ps, int mode, int M) {
     } else {
       for (int k = 0; k < n; ++k) w.push_back(dht ? std::complex<ld>(0.5L, 0.5L) : expi_pi(k, 2 * (int64_t)n));
     }
-    rc = upload_sm_vec(P, key, w, 1);
+    rc = upload_shifted(P, key, w, 1);
     if (rc) return rc;
   }
   ps.d23_tab = P->tables[key];

@@ -96,14 +96,23 @@ struct xf_tw {
 
 // shifts 1 .. kXfShifts: one table each, one after the other
 constexpr int kXfShifts = 3;
-// appends the entry of w (parts of magnitude at most 1, of any precision) for
-// the shift s to a table of 32-bit words
-template <typename V, typename C>
-inline void push_xf_twiddle(V& t, const C& w, int s) {
+// a twiddle (parts of magnitude at most 1) as doubles and what they leave; once
+// for all shifts, since the Arm host's long double is software
+struct xf_tw_parts {
+  double hi[2], lo[2];
+};
+template <typename C>
+inline xf_tw_parts split_twiddle(const C& w) {
   const auto x = w.real(), y = w.imag();
+  const double h[2] = {(double)x, (double)y};
+  return {{h[0], h[1]}, {(double)(x - h[0]), (double)(y - h[1])}};
+}
+// appends the entry of w for the shift s to a table of 32-bit words
+template <typename V>
+inline void push_xf_twiddle(V& t, const xf_tw_parts& w, int s) {
   const double q = (double)(1ll << (32 - s));
-  const double c[2] = {(double)x * q, (double)y * q};
-  const double rest[2] = {(double)(x - (double)x) * q, (double)(y - (double)y) * q};
+  const double c[2] = {w.hi[0] * q, w.hi[1] * q};
+  const double rest[2] = {w.lo[0] * q, w.lo[1] * q};
   float o[2];
   for (int i = 0; i < 2; ++i) {
     const long long r = (long long)(c[i] < 0 ? c[i] - 0.5 : c[i] + 0.5);
@@ -115,6 +124,11 @@ inline void push_xf_twiddle(V& t, const C& w, int s) {
   }
   t.push_back(o[0]);
   t.push_back(o[1]);
+}
+
+template <typename V, typename C>
+inline void push_xf_twiddle(V& t, const C& w, int s) {
+  push_xf_twiddle(t, split_twiddle(w), s);
 }
 
 // (re, im) times w (CONJ: times its conjugate), in units 2^s times larger.

@@ -817,14 +817,14 @@ static int sm_best_pitch(int M, int w, int q, int r0, int ebytes) {
 // (few): launch latency sets their time, and the plans that ask for those
 // kernels by name in tests have few lines.  Measured round trips, Bluestein or
 // (*) mixed-radix tile against this one: Float64 RFFT 100^3 0.213 -> 0.082 ms,
-// 240^3 1.98 -> 0.64, 360^3 9.73 -> 2.42, *384^3 3.97 -> 2.65, FFT *96^3 0.286
+// 240^3 1.98 -> 0.64, 360^3 9.73 -> 2.42, *384^3 3.97 -> 2.36, FFT *96^3 0.286
 // -> 0.100, *24^3 0.139 -> 0.045, 1000^2 0.260 -> 0.124; Float32 RFFT 360^3 3.45 -> 0.83, 120^3 0.088 -> 0.069,
 // 50x60x70 0.040 -> 0.041, FFT 200^3 0.629 -> 0.274.
 //
 // The tile: w lines and a butterfly step q (w q threads), by the share of
 // threads that have work in every stage, the threads in flight on an SM, 64
-// contiguous bytes at least on a strided axis, 8 lines side by side for the
-// banks, and the last wave.
+// contiguous bytes at least on a strided axis, 8 lines side by side, and the
+// last wave.
 static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
   taken = false;
   const int M = ps.M;
@@ -862,7 +862,11 @@ static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
       if (occ < 768) cost *= std::sqrt(768 / occ);
       const int chunk = w * 2 * P->rb;  // contiguous bytes on a strided axis
       if (strided && chunk < 128) cost *= chunk >= 64 ? 1.1 : 1.1 * 64 / chunk;
-      if (w < 8) cost *= 1.2;  // bank conflicts of less than 8 lines side by side
+      // fewer than 8 lines side by side share less of each twiddle load; four
+      // Float64 lines (64-byte rows) lose little and leave room for more tiles
+      // (384^3 round trip 2634 -> 2355 us against 1.2, where none at all makes
+      // 240^3 630 -> 669 us)
+      if (w < 8) cost *= w >= 4 && f64 ? 1.07 : 1.2;
       const double waves = (double)((ncl + w - 1) / w * outer) / (152.0 * ctas);
       cost *= std::ceil(waves) / waves * ((double)((ncl + w - 1) / w * w) / ncl);
       if (cost < best) { best = cost; tw = w; k = q; }

@@ -324,7 +324,7 @@ inline void stage_twiddles(int logm, int lp, F f) {
 
 // v times the conjugate of (SIGN > 0), or the twiddle table's entry m (fx
 // tables hold the pass's sign already)
-template <typename R, int SIGN>
+template <typename R, int SIGN, bool ROUND = false>
 __device__ __forceinline__ Cx<R> tw_mul(Cx<R> v, const void* tw, int m) {
   if constexpr (std::is_same<R, fx>::value) {
     const int4 q = __ldg(reinterpret_cast<const int4*>(tw) + m);
@@ -332,7 +332,7 @@ __device__ __forceinline__ Cx<R> tw_mul(Cx<R> v, const void* tw, int m) {
     return v;
   } else if constexpr (std::is_same<R, xf>::value) {  // the product in units 2^s times larger
     const int4 q = __ldg(reinterpret_cast<const int4*>(tw) + m);
-    xf_twiddle<(SIGN > 0)>(v.re, v.im, xf_tw{q.x, q.y, __int_as_float(q.z), __int_as_float(q.w)});
+    xf_twiddle<(SIGN > 0), ROUND>(v.re, v.im, xf_tw{q.x, q.y, __int_as_float(q.z), __int_as_float(q.w)});
     return v;
   } else {
     Cx<R> w = ldg_tw<R>(tw, m);
@@ -457,9 +457,8 @@ __device__ __forceinline__ unsigned line_max_get(unsigned m, const unsigned* red
 // against 7 per 16 lanes and radix-8 stage; the Float32 passes are bound by
 // these lookups and the exchanges (round trips: 512^3 Float32 1.41 -> 1.26 ms,
 // 1024^3 13.2 -> 11.0 ms, 512^3 Float64 4.40 -> 4.14 ms).  R = xf: the line's
-// shifts (pfgb_xf.cuh) are added to shifts, HEAD more bits are kept free; red:
-// one word a thread.
-template <typename R, int LOGM, int SIGN, int OP, int P, bool ZH, int HEAD = 0>
+// shifts (pfgb_xf.cuh) are added to shifts; red: one word a thread.
+template <typename R, int LOGM, int SIGN, int OP, int P, bool ZH>
 __device__ __forceinline__ void stages_core(Cx<R> (&v)[P], Cx<R>* z, int p, int b, const void* tw,
                                             bool lanes_across_lines, unsigned* red, int& shifts) {
   constexpr bool XF = std::is_same<R, xf>::value;
@@ -477,13 +476,21 @@ __device__ __forceinline__ void stages_core(Cx<R> (&v)[P], Cx<R>* z, int p, int 
   for (int s = 0; s < NST; ++s) {
     const bool last = (s == NST - 1);
     const void* tws = XF && s > 0 ? reinterpret_cast<const int4*>(tw) + (sh - 1) * (M - P) : tw;
+    // (folded: the loop is unrolled)
+    const bool round = XF && xf_rounds(LOGM) && s + 2 >= NST;
+    auto twiddle = [&](const Cx<R>& x, int m) {
+      return round ? tw_mul<R, SIGN, true>(x, tws, m) : tw_mul<R, SIGN>(x, tws, m);
+    };
+    auto down = [&](const Cx<xf>& x) {
+      return round ? mk(xf_shift<true>(x.re, sh), xf_shift<true>(x.im, sh)) : mk(xf_shift(x.re, sh), xf_shift(x.im, sh));
+    };
     if (s < SP) {
       const int j = b & (Ls - 1);
       if (Ls > 1) {
         const int e0 = Ls - P + j;  // the stage's first entry (Ls - P), lane j
 #pragma unroll
-        for (int r = 1; r < P; ++r) v[r] = tw_mul<R, SIGN>(v[r], tws, e0 + (r - 1) * Ls);
-        if constexpr (XF) v[0] = mk(xf_shift(v[0].re, sh), xf_shift(v[0].im, sh));
+        for (int r = 1; r < P; ++r) v[r] = twiddle(v[r], e0 + (r - 1) * Ls);
+        if constexpr (XF) v[0] = down(v[0]);
       }
       if constexpr (P == 16) dft16<SIGN>(v);
       else if (ZH && s == 0) dft8_zh<SIGN>(v);
@@ -502,9 +509,8 @@ __device__ __forceinline__ void stages_core(Cx<R> (&v)[P], Cx<R>* z, int p, int 
       for (int r1 = 0; r1 < G; ++r1) {
         const int beta = Ls - P + b + r1 * T;
 #pragma unroll
-        for (int q = 1; q < RS; ++q)
-          v[r1 + q * G] = tw_mul<R, SIGN>(v[r1 + q * G], tws, beta + (q - 1) * (M / RS));
-        if constexpr (XF) v[r1] = mk(xf_shift(v[r1].re, sh), xf_shift(v[r1].im, sh));
+        for (int q = 1; q < RS; ++q) v[r1 + q * G] = twiddle(v[r1 + q * G], beta + (q - 1) * (M / RS));
+        if constexpr (XF) v[r1] = down(v[r1]);
         if constexpr (RS == 2) {
           dft2<SIGN>(v[r1], v[r1 + G]);
         } else if constexpr (RS == 4) {
@@ -531,21 +537,21 @@ __device__ __forceinline__ void stages_core(Cx<R> (&v)[P], Cx<R>* z, int p, int 
       }
       line_sync<R, LOGM, OP, P>(lanes_across_lines, p);
       const int zr = sidx<R, LOGM, OP>(p, b);
-#pragma unroll
-      for (int r = 0; r < P; ++r) v[r] = xld<R, LOGM, OP>(z, zr + padded<R, LOGM>(r * T));
-      if constexpr (XF) {
+      if constexpr (XF) {  // before the reads (after them: 512^3 Float64 3384 against 3265 us)
         lmax = line_max_get<LOGM, OP>(lmax, red, lanes_across_lines, p);
-        sh = xf_stage_shift(lmax, (s + 1 < SP ? 3 : REM) + HEAD);
+        sh = xf_stage_shift(lmax, s + 1 < SP ? 3 : REM);
         shifts += sh;
       }
+#pragma unroll
+      for (int r = 0; r < P; ++r) v[r] = xld<R, LOGM, OP>(z, zr + padded<R, LOGM>(r * T));
       line_sync<R, LOGM, OP, P>(lanes_across_lines, p);
     }
   }
 }
 
 // A double-float line's values in xf, scaled by the line's largest high part;
-// returns its biased float exponent (at least 27, plus HEAD).
-template <int LOGM, int OP, int NIN, int HEAD = 0>
+// returns its biased float exponent (at least 27).
+template <int LOGM, int OP, int NIN>
 __device__ __forceinline__ unsigned line_to_xf(const Cx<dd> (&v)[8], Cx<xf> (&x)[8], unsigned* red,
                                                bool lanes_across_lines, int p) {
   float mf = 0.0f;  // (a NaN is in the fractions: xf_line_exp)
@@ -553,7 +559,7 @@ __device__ __forceinline__ unsigned line_to_xf(const Cx<dd> (&v)[8], Cx<xf> (&x)
   for (int r = 0; r < NIN; ++r) mf = fmaxf(fmaxf(mf, fabsf(v[r].re.h)), fabsf(v[r].im.h));
   const unsigned m = line_max_put<LOGM, OP>(__float_as_uint(mf), red, lanes_across_lines, p);
   if constexpr (LOGM > 3) line_sync<dd, LOGM, OP>(lanes_across_lines, p);
-  const unsigned e = xf_line_exp(line_max_get<LOGM, OP>(m, red, lanes_across_lines, p)) + HEAD;
+  const unsigned e = xf_line_exp(line_max_get<LOGM, OP>(m, red, lanes_across_lines, p));
   const float f = xf_scale_in(e);
 #pragma unroll
   for (int r = 0; r < NIN; ++r) x[r] = mk(dd2xf(v[r].re, f), dd2xf(v[r].im, f));
@@ -572,7 +578,7 @@ __device__ __forceinline__ void fast_stages(Cx<R> (&v)[P], Cx<R>* z, int p, int 
     const unsigned e = line_to_xf<LOGM, OP, ZH ? P / 2 : P>(v, x, red[0], lanes_across_lines, p);
     stages_core<xf, LOGM, SIGN, OP, P, ZH>(x, reinterpret_cast<Cx<xf>*>(z), p, b, tw, lanes_across_lines, red[1],
                                            shifts);
-    const unsigned ue = xf_unit_exp(e) + (unsigned)shifts;
+    const int ue = xf_unit_exp(e) + shifts;
 #pragma unroll
     for (int r = 0; r < P; ++r) v[r] = mk(xf2dd(x[r].re, ue), xf2dd(x[r].im, ue));
   } else {
@@ -1517,6 +1523,11 @@ __device__ __forceinline__ void fast_tile_store(const FastArgs& a, int64_t bid, 
   }
 }
 
+// (f + g) / 2: a r2c line's outputs may fill the whole range
+__device__ __forceinline__ Cx<xf> xf_half_sum(Cx<xf> f, Cx<xf> g) {
+  return mk(xf_half_sum(f.re, g.re), xf_half_sum(f.im, g.im));
+}
+
 // Operations of a double-float pass whose tile stays in xf from the load to
 // the store (fast_tile_xf); the others convert around their stages.
 __host__ __device__ constexpr bool fast_xf_op(int op) { return op == OP_C2C || op == OP_R2C || op == OP_C2R; }
@@ -1535,8 +1546,6 @@ __device__ __forceinline__ void fast_tile_xf(const FastArgs& a, int64_t bid, Cx<
   constexpr int T = M / 8;
   constexpr int TW = fast_tw<dd>(LOGM, OP);
   constexpr int TH = fast_threads<dd>(LOGM, OP);
-  // the r2c split adds two outputs of a line: one more bit kept free
-  constexpr int HEAD = OP == OP_R2C ? 1 : 0;
   const int tid = threadIdx.x;
   const bool lanes = a.lmap_tile != 0;
   int p, b;
@@ -1576,32 +1585,32 @@ __device__ __forceinline__ void fast_tile_xf(const FastArgs& a, int64_t bid, Cx<
     const float fs = xf_frac_scale(s.emax);
 #pragma unroll
     for (int r = 0; r < 8; ++r)
-      x[r] = mk(d2xf<26 - HEAD>(raw[r].x, s.emax, fs), d2xf<26 - HEAD>(raw[r].y, s.emax, fs));
-    ue = 101 + HEAD;
+      x[r] = mk(d2xf<26>(raw[r].x, s.emax, fs), d2xf<26>(raw[r].y, s.emax, fs));
+    ue = 101;
     if (OP == OP_C2C && a.deriv == 1) {
       Cx<dd> v[8];
 #pragma unroll
       for (int r = 0; r < 8; ++r) {
         const int64_t idx = a.deriv_role == 0 ? (int64_t)(b + r * T) : a.deriv_role == 1 ? s.t0 + p : s.didx;
-        v[r] = mul_ik(mk(xf2dd(x[r].re, 101u), xf2dd(x[r].im, 101u)), idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
+        v[r] = mul_ik(mk(xf2dd(x[r].re, 101), xf2dd(x[r].im, 101)), idx, a.deriv_half, a.deriv_n, a.k0_h, a.k0_l);
       }
-      ue = (int)xf_unit_exp(line_to_xf<LOGM, OP, 8>(v, x, red[1], lanes, p));
+      ue = xf_unit_exp(line_to_xf<LOGM, OP, 8>(v, x, red[1], lanes, p));
       line_sync<dd, LOGM, OP>(lanes, p);  // red[1] is used again below
     }
   } else {
     Cx<dd> v[8];
     fast_tile_load<dd, LOGM, SIGN, OP, IOM>(a, bid, src, ssa, sst, p, b, s, v);
-    ue = (int)xf_unit_exp(line_to_xf<LOGM, OP, 8, HEAD>(v, x, red[0], lanes, p));
+    ue = xf_unit_exp(line_to_xf<LOGM, OP, 8>(v, x, red[0], lanes, p));
   }
   int shifts = 0;
-  stages_core<xf, LOGM, SIGN, OP, 8, false, HEAD>(x, reinterpret_cast<Cx<xf>*>(z), p, b, a.tw, lanes, red[1], shifts);
+  stages_core<xf, LOGM, SIGN, OP, 8, false>(x, reinterpret_cast<Cx<xf>*>(z), p, b, a.tw, lanes, red[1], shifts);
   ue += shifts;
 
   // ---- store ----
   if (OP == OP_C2C && a.deriv == 2) {
     Cx<dd> v[8];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) v[r] = mk(xf2dd(x[r].re, (unsigned)ue), xf2dd(x[r].im, (unsigned)ue));
+    for (int r = 0; r < 8; ++r) v[r] = mk(xf2dd(x[r].re, ue), xf2dd(x[r].im, ue));
     if (b == 0) lexp[p] = s.emax;
     fast_tile_store<dd, LOGM, SIGN, OP, IOM>(a, bid, p, b, s, v, z, lexp);
     return;
@@ -1613,7 +1622,7 @@ __device__ __forceinline__ void fast_tile_xf(const FastArgs& a, int64_t bid, Cx<
     xf2d(y, off, o.x, o.y);
     return o;
   };
-  auto to_dd4 = [](Cx<xf> y, int u) { return st_dd4(mk(xf2dd(y.re, (unsigned)u), xf2dd(y.im, (unsigned)u))); };
+  auto to_dd4 = [](Cx<xf> y, int u) { return st_dd4(mk(xf2dd(y.re, u), xf2dd(y.im, u))); };
   const int off = ue + s.emax_out - 254 + a.scale_xe;
   if (a.store_direct && OP != OP_R2C) {
     if constexpr (OP == OP_C2C) {
@@ -1646,8 +1655,9 @@ __device__ __forceinline__ void fast_tile_xf(const FastArgs& a, int64_t bid, Cx<
     for (int r = 0; r < 8; ++r) zw[padded<xf, LOGM>(r * T)] = x[r];
   }
   if (b == 0) {
-    lue[p] = ue;
-    loff[p] = off;
+    constexpr int halved = OP == OP_R2C ? 1 : 0;
+    lue[p] = ue + halved;
+    loff[p] = off + halved;
   }
   __syncthreads();
   if constexpr (OP == OP_C2C) {
@@ -1668,7 +1678,7 @@ __device__ __forceinline__ void fast_tile_xf(const FastArgs& a, int64_t bid, Cx<
       if (a.out_tfast) { q = e % TW; k = e / TW; } else { k = e % m; q = e / m; }
       const Cx<xf> f = zx[sidx<xf, LOGM, OP>(q, k)];
       const Cx<xf> g = conj(zx[sidx<xf, LOGM, OP>(q, k == 0 ? 0 : M - k)]);
-      const Cx<xf> A = f + g, B = mul_mi(f - g);  // (the factor 1/2: emax_shift)
+      const Cx<xf> A = xf_half_sum(f, g), B = mul_mi(xf_half_sum(f, -g));  // (the split's own 1/2: emax_shift)
       const int64_t o = s.ooff + (int64_t)k * a.out_sa + (int64_t)(2 * q) * a.out_st;
       if constexpr (OUT_DD) {
         const int u = lue[q];

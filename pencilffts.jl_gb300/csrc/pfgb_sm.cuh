@@ -30,15 +30,7 @@ constexpr int kSmThreads = 256;
 
 // a c for a compile-time constant |c| <= 1, in a's unit
 __device__ __forceinline__ float mulc(float a, double c) { return a * (float)c; }
-__device__ __forceinline__ xf mulc(xf a, double c) {
-  const int base = c > 0.5 ? 1 : c < -0.5 ? -1 : 0;
-  const double r = (c - base) * 4294967296.0;
-  const int w = (int)(r < -2147483648.0 ? -2147483648.0 : r > 2147483647.0 ? 2147483647.0 : r);
-  const uint64_t p = (uint64_t)((int64_t)a.h * w);
-  const float f = f_fma(xf_i2f(a.h), (float)((r - w) * 0x1p-32), f_mul(a.l, (float)c));
-  const int b = base > 0 ? a.h : base < 0 ? -a.h : 0;
-  return xf(b + (int)(p >> 32), xf_frac((uint32_t)p, f));
-}
+__device__ __forceinline__ xf mulc(xf a, double c) { return xf_mulc(a, c); }
 template <typename R>
 __device__ __forceinline__ Cx<R> mulc(Cx<R> a, double c) { return mk(mulc(a.re, c), mulc(a.im, c)); }
 
@@ -309,12 +301,12 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
   using MR = typename std::conditional<XF, double, float>::type;
   using MC = typename std::conditional<XF, double2, float2>::type;
   // xf: bits of the largest component at the first stage, below 27 by one for
-  // the r2c split's sum and for c2r's sum of two spectra
+  // c2r's sum of two spectra (the r2c split halves its sums)
   constexpr bool R2R = OP == OP_R2R_C || OP == OP_R2R_R;
   constexpr bool CIN = OP == OP_C2C || OP == OP_R2R_C;  // complex elements in and out
   // (D2: for its sum of two outputs; D4: one above, its first twiddles shift by one)
-  const int head = OP == OP_R2C || (R2R && a.sm_mode == SM_D2) ? 1 : 0;
-  const int bits = !R2R ? 26 - (OP == OP_C2C ? 0 : 1) : a.sm_mode == SM_D2 ? 25 : a.sm_mode == SM_D4 ? 27 : 26;
+  const int head = R2R && a.sm_mode == SM_D2 ? 1 : 0;
+  const int bits = !R2R ? 26 - (OP == OP_C2R ? 1 : 0) : a.sm_mode == SM_D2 ? 25 : a.sm_mode == SM_D4 ? 27 : 26;
   constexpr bool packed = !CIN;
   __shared__ unsigned lm[kSmStages][kSmLines];  // xf: per line, the input's largest exponent, then the stages' components
   __shared__ int loff[kSmLines];
@@ -559,8 +551,7 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
     if constexpr (XF) atomicMax(&lm[s][t.p], t.m);
     __syncthreads();
     if constexpr (XF) {
-      const int r = a.sm_r[s];
-      t.sh = xf_stage_shift(lm[s][t.p], (r <= 2 ? 1 : r <= 4 ? 2 : 3) + head);
+      t.sh = xf_shift_of(xf_excess(lm[s][t.p], a.sm_r[s]) + head);
       shifts += t.sh;
     }
     t.zi = za + t.p * pitch;
@@ -573,8 +564,8 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
   }
   if constexpr (XF && R2R) shifts += a.sm_mode == SM_D2 || a.sm_mode == SM_D4 ? 1 : 0;  // twiddles after the last
   if constexpr (XF) {
-    // the unit's exponent with the line's (r2c: its factor 1/2), and the normalisation's
-    if (t.b0 == 0) loff[t.p] = 127 - bits + shifts + (int)lm[0][t.p] + a.emax_shift - 254 + a.scale_xe - (OP == OP_R2C ? 1 : 0);
+    // the unit's exponent with the line's, and the normalisation's
+    if (t.b0 == 0) loff[t.p] = 127 - bits + shifts + (int)lm[0][t.p] + a.emax_shift - 254 + a.scale_xe;
   }
   __syncthreads();
 
@@ -626,8 +617,13 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
         reinterpret_cast<MC*>(a.out)[w.off] = y;
       } else if constexpr (OP == OP_R2C) {
         const Cx<R> f = zl[k], g = conj(zl[k == 0 ? 0 : M - k]);
-        Cx<R> A = f + g, B = mul_mi(f - g);
-        if constexpr (!XF) {
+        Cx<R> A, B;
+        if constexpr (XF) {
+          A = xf_half_sum(f, g);
+          B = mul_mi(xf_half_sum(f, -g));
+        } else {
+          A = f + g;
+          B = mul_mi(f - g);
           A = mk(half(A.re), half(A.im));
           B = mk(half(B.re), half(B.im));
         }

@@ -6,26 +6,32 @@
 // h a 32-bit integer count of the line's unit q, l a float holding the
 // fraction below it (|l| of a few units).  Sums are one integer and one float
 // addition, exact in h.  A product with a twiddle w, |w| <= 1, is a 32 x 32
-// -> 64-bit integer product with W = round(w 2^(32 - s)): its high word is the
-// new h, in units 2^s q, its low word the new fraction; the rest of w (o =
-// w 2^(32 - s) - W) and the product of l go into the fraction in float.
+// -> 64-bit integer product with W = round(w 2^(32 - s)): its high word, to
+// nearest, is the new h, in units 2^s q, its low word the new fraction; the
+// rest of w (o = w 2^(32 - s) - W) and the product of l go into the fraction in
+// float.
 //
-// Range: the line's complex values stay within 2^27.5 units in modulus before
-// a radix-8 butterfly and so within 2^30.5 after it: h cannot overflow.  The
-// line enters with components below 2^27 (its largest in [2^26, 2^27)), and
-// the twiddles of each later stage carry the shift s = 1, 2 or 3 that the
-// line's largest component after the previous butterfly asks for
-// (xf_stage_shift; s = 3 always suffices).  The tables hold all three forms,
-// so the shift costs no instruction.
+// Range: a line's complex values stay within 0.95 2^31 / r units in modulus
+// before a radix-r butterfly, r <= 8, and so within 0.95 2^31 after it: h cannot
+// overflow.  The line enters with components below 2^27 (its largest in
+// [2^26, 2^27)), and the twiddles of each later stage carry the shift s = 1, 2
+// or 3 that the line's largest component after the previous butterfly asks for
+// (xf_excess, xf_shift_of; s = 3 always suffices).  The tables hold all three
+// forms, so the shift costs no instruction.
 //
-// Cost: 205 to 265 instructions a point in a 512-point pass, where the dd
-// stages took 277 to 383; 512^3 Float64 round trip 4.14 -> 3.35 ms, 256^3
-// complex 0.945 -> 0.741 ms.
+// Cost: 512^3 Float64 round trip 4.14 ms with dd stages, 3.28 ms with these;
+// 256^3 complex 0.945 and 0.725 ms.
 //
-// Precision: each operation rounds the fraction at about 2^-24 unit, and the
-// line's largest value stays near 2^26 units or above, whatever the data (a
-// fixed s = 3 would leave lines of few non-zero points, which do not grow, at
-// 2^-45).
+// Precision: each operation rounds the fraction at about 2^-24 unit, whatever the
+// value, where a dd stage's error follows the single value.  Lines of noise have
+// a third of dd's error.  The line that can lose is the one whose sum grows with
+// its length (a large mean, a ramp): its small outputs carry the error that goes
+// with the large one, as sqrt(M).  tests/test_xf_lines.py holds such lines below dd's
+// error at all lengths; what that took, as multiples of dd's error:
+//   4096 points, mean 10 and noise: 1.7 with high words rounded down in every
+//     stage and a bit of the range unused, 0.8 as it is (xf_rounds, xf_excess);
+//   512 points, mean 1000 and noise, r2c: 1.6 with one bit of the range kept free
+//     for the split's sum, 0.8 with the sum halved (xf_half_sum).
 #pragma once
 
 #include <stdint.h>
@@ -54,16 +60,6 @@ PFGB_HD xf operator+(xf a, xf b) { return xf(a.h + b.h, f_add(a.l, b.l)); }
 PFGB_HD xf operator-(xf a, xf b) { return xf(a.h - b.h, f_sub(a.l, b.l)); }
 PFGB_HD xf operator-(xf a) { return xf(-a.h, -a.l); }
 
-// u 2^-32 + f for the low word u of a product whose high word was rounded down
-// (to nearest, the rounding constant would cost register moves: 512^3 Float64
-// 3.46 against 3.35 ms)
-PFGB_HD float xf_frac(uint32_t u, float f) {
-#if defined(__CUDA_ARCH__)
-  return f_fma(__uint2float_rn(u), 0x1p-32f, f);
-#else
-  return f_fma((float)u, 0x1p-32f, f);
-#endif
-}
 PFGB_HD float xf_i2f(int x) {
 #if defined(__CUDA_ARCH__)
   return __int2float_rn(x);
@@ -72,12 +68,53 @@ PFGB_HD float xf_i2f(int x) {
 #endif
 }
 
+// u 2^-32 + f for the low word u of a product whose high word was rounded down
+PFGB_HD float xf_frac(uint32_t u, float f) {
+#if defined(__CUDA_ARCH__)
+  return f_fma(__uint2float_rn(u), 0x1p-32f, f);
+#else
+  return f_fma((float)u, 0x1p-32f, f);
+#endif
+}
+// p 2^-32 + f for a product p: its high word rounded down, or to nearest
+// (ROUND: the low word is a signed fraction then, and its top bit the carry).
+// Fractions rounded down do not cancel in the butterflies' sums: 1.2 to 1.9
+// times the error.
+template <bool ROUND>
+PFGB_HD xf xf_product(uint64_t p, float f) {
+  const uint32_t u = (uint32_t)p;
+  if (ROUND) return xf((int)(p >> 32) + (int)(u >> 31), f_fma(xf_i2f((int)u), 0x1p-32f, f));
+  return xf((int)(p >> 32), xf_frac(u, f));
+}
+// Power-of-two lines that need it, in their last two stages (an earlier stage's
+// error counts an eighth of the next one's): 4096^2 complex round trip 873 us
+// without, 891 us, 930 us with every stage rounded.  Smooth lines, up to 2048
+// points but for 2560, stay below dd's error without.
+PFGB_HD constexpr bool xf_rounds(int logm) { return logm > 10; }
+
 // a c, in a's unit
 PFGB_HD xf operator*(xf a, xf c) {
   const float cf = f_fma((float)c.h, 0x1p-32f, 1.0f);
   const uint64_t p = (uint64_t)((int64_t)a.h * c.h);
   const float f = f_fma(xf_i2f(a.h), c.l * 0x1p-32f, f_mul(a.l, cf));
   return xf(a.h + (int)(p >> 32), xf_frac((uint32_t)p, f));
+}
+
+// a c for a compile-time constant |c| <= 1, in a's unit
+PFGB_HD xf xf_mulc(xf a, double c) {
+  const int base = c > 0.5 ? 1 : c < -0.5 ? -1 : 0;
+  const double r = (c - base) * 4294967296.0;
+  const int w = (int)(r < -2147483648.0 ? -2147483648.0 : r > 2147483647.0 ? 2147483647.0 : r);
+  const uint64_t p = (uint64_t)((int64_t)a.h * w);
+  const float f = f_fma(xf_i2f(a.h), (float)((r - w) * 0x1p-32), f_mul(a.l, (float)c));
+  const int b = base > 0 ? a.h : base < 0 ? -a.h : 0;
+  return xf(b + (int)(p >> 32), xf_frac((uint32_t)p, f));
+}
+
+// (a + b) / 2 where a + b may be beyond 2^31
+PFGB_HD xf xf_half_sum(xf a, xf b) {
+  const int x = a.h ^ b.h;
+  return xf((a.h & b.h) + (x >> 1), f_fma(f_add(a.l, b.l), 0.5f, x & 1 ? 0.5f : 0.0f));
 }
 
 // a c for a factor c in [1/2, 1) given as w = round(c 2^31), o = (c 2^31 - w)
@@ -132,7 +169,7 @@ inline void push_xf_twiddle(V& t, const C& w, int s) {
 }
 
 // (re, im) times w (CONJ: times its conjugate), in units 2^s times larger.
-template <bool CONJ>
+template <bool CONJ, bool ROUND = false>
 PFGB_HD void xf_twiddle(xf& re, xf& im, xf_tw w) {
   const int wi = CONJ ? -w.wi : w.wi, mwi = CONJ ? w.wi : -w.wi;
   const float oi = CONJ ? -w.oi : w.oi;
@@ -141,34 +178,41 @@ PFGB_HD void xf_twiddle(xf& re, xf& im, xf_tw w) {
   const float wrf = xf_i2f(w.wr), wif = xf_i2f(wi), hr = xf_i2f(re.h), hi = xf_i2f(im.h);
   const float ar = f_fma(re.l, wrf, f_fma(-im.l, wif, f_fma(-hi, oi, f_mul(hr, w.orr))));
   const float ai = f_fma(re.l, wif, f_fma(im.l, wrf, f_fma(hi, w.orr, f_mul(hr, oi))));
-  re = xf((int)(pr >> 32), xf_frac((uint32_t)pr, f_mul(ar, 0x1p-32f)));
-  im = xf((int)(pi >> 32), xf_frac((uint32_t)pi, f_mul(ai, 0x1p-32f)));
+  re = xf_product<ROUND>(pr, f_mul(ar, 0x1p-32f));
+  im = xf_product<ROUND>(pi, f_mul(ai, 0x1p-32f));
 }
 
 // a in units 2^s times larger
+template <bool ROUND = false>
 PFGB_HD xf xf_shift(xf a, int s) {
 #if defined(__CUDA_ARCH__)
   const float f = __uint_as_float((unsigned)(127 - s) << 23);
 #else
   const float f = 1.0f / (float)(1 << s);
 #endif
+  if (ROUND) {
+    const int h = (a.h + (1 << (s - 1))) >> s;
+    return xf(h, f_mul(f, f_add(a.l, xf_i2f(a.h - (h << s)))));
+  }
   return xf(a.h >> s, f_mul(f, f_add(a.l, xf_i2f(a.h & ((1 << s) - 1)))));
 }
-
-// Shift of the twiddles before a butterfly of radix 2^lr, from the line's
-// largest h or ~h: components below 2^(30 - lr) units afterwards, so that the
-// butterfly's sums stay below 2^31 (complex moduli sqrt 2 times the
-// components'), within 1 .. 3.  With 31 bits (moduli up to 2^30.5) three are
-// enough.  A line that keeps one more bit free passes lr + 1.
-PFGB_HD int xf_stage_shift(unsigned m, int lr) {
+// Bits of a line with largest h or ~h m beyond what a butterfly of radix r <= 8
+// takes: 1.5 r m (1.5 and not sqrt 2 for the complex moduli, and for what the
+// fractions add) is to stay below 2^31.
+PFGB_HD int xf_bits(unsigned m) {
 #if defined(__CUDA_ARCH__)
-  const int bl = 32 - __clz((int)m);
+  return 32 - __clz((int)m);
 #else
-  const int bl = m ? 32 - __builtin_clz(m) : 0;
+  return m ? 32 - __builtin_clz(m) : 0;
 #endif
-  const int s = bl - (30 - lr);
-  return s < 1 ? 1 : s > kXfShifts ? kXfShifts : s;
 }
+PFGB_HD int xf_excess(unsigned m, int r) { return xf_bits(((m >> 4) + 1u) * (3u * (unsigned)r)) - 28; }
+// Shift of the twiddles before that butterfly, within 1 .. 3: with moduli up to
+// 0.95 2^31 three are enough.
+PFGB_HD int xf_shift_of(int excess) { return excess < 1 ? 1 : excess > kXfShifts ? kXfShifts : excess; }
+// r = 2^lr: one instruction less
+PFGB_HD int xf_excess_pow2(unsigned m, int lr) { return xf_bits(m + (m >> 1)) - 31 + lr; }
+PFGB_HD int xf_stage_shift(unsigned m, int lr) { return xf_shift_of(xf_excess_pow2(m, lr)); }
 
 // A dd line in xf units: from the float bits m of its largest |high part|, the
 // scale 2^(153 - e), e the biased exponent of m, at least 27 (a line below
@@ -185,7 +229,7 @@ __device__ __forceinline__ float xf_scale_in(unsigned e) {
   return __uint_as_float((280u - e) << 23);
 }
 // biased float exponent of the unit in the dd line's scale, before any shift
-__device__ __forceinline__ unsigned xf_unit_exp(unsigned e) { return min(e, 254u) - 26u; }
+__device__ __forceinline__ int xf_unit_exp(unsigned e) { return (int)min(e, 254u) - 26; }
 
 __device__ __forceinline__ xf dd2xf(dd a, float f) {
   const float hs = f_mul(a.h, f);
@@ -197,9 +241,10 @@ __device__ __forceinline__ void xf_split(xf a, float& hi, float& lo) {
   hi = __int2float_rn(a.h);
   lo = f_add(a.l, __int2float_rn(a.h - __float2int_rn(hi)));
 }
-// a 2^(ue - 127): ue the unit's biased exponent
-__device__ __forceinline__ dd xf2dd(xf a, unsigned ue) {
-  const float g = __uint_as_float(ue << 23);
+// a 2^(ue - 127): ue the unit's biased exponent, above -23 (below 1 for lines
+// near the bottom of the dd range that went up)
+__device__ __forceinline__ dd xf2dd(xf a, int ue) {
+  const float g = __uint_as_float(ue > 0 ? (unsigned)ue << 23 : 0x800000u >> (1 - ue));
   float hi, lo;
   xf_split(a, hi, lo);
   return dd(f_mul(hi, g), f_mul(lo, g));

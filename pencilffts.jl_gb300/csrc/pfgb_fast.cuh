@@ -539,8 +539,17 @@ __device__ __forceinline__ void stages_core(Cx<R> (&v)[P], Cx<R>* z, int p, int 
       const int zr = sidx<R, LOGM, OP>(p, b);
       if constexpr (XF) {  // before the reads (after them: 512^3 Float64 3384 against 3265 us)
         lmax = line_max_get<LOGM, OP>(lmax, red, lanes_across_lines, p);
-        sh = xf_stage_shift(lmax, s + 1 < SP ? 3 : REM);
+        const int lr = s + 1 < SP ? 3 : REM;
+        sh = xf_stage_shift(lmax, lr);
         shifts += sh;
+        if (const int up = xf_ups(LOGM) ? xf_up_of(xf_excess_pow2(lmax, lr)) : 0) {  // in place: no other thread reads this one's inputs
+#pragma unroll 1
+          for (int r = 0; r < P; ++r) {
+            Cx<R>& x = z[zr + padded<R, LOGM>(r * T)];
+            x = mk(xf_up(x.re, up), xf_up(x.im, up));
+          }
+          shifts -= up;
+        }
       }
 #pragma unroll
       for (int r = 0; r < P; ++r) v[r] = xld<R, LOGM, OP>(z, zr + padded<R, LOGM>(r * T));

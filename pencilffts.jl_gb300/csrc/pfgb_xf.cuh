@@ -17,7 +17,9 @@
 // [2^26, 2^27)), and the twiddles of each later stage carry the shift s = 1, 2
 // or 3 that the line's largest component after the previous butterfly asks for
 // (xf_excess, xf_shift_of; s = 3 always suffices).  The tables hold all three
-// forms, so the shift costs no instruction.
+// forms, so the shift costs no instruction.  A line that grew too little for
+// s = 1 (few non-zero points, small radices) goes up by some bits first
+// (xf_up_of).
 //
 // Cost: 512^3 Float64 round trip 4.14 ms with dd stages, 3.28 ms with these;
 // 256^3 complex 0.945 and 0.725 ms.
@@ -26,12 +28,14 @@
 // value, where a dd stage's error follows the single value.  Lines of noise have
 // a third of dd's error.  The line that can lose is the one whose sum grows with
 // its length (a large mean, a ramp): its small outputs carry the error that goes
-// with the large one, as sqrt(M).  tests/test_xf_lines.py holds such lines below dd's
-// error at all lengths; what that took, as multiples of dd's error:
+// with the large one, as sqrt(M).  tests/test_xf_lines.py holds such lines, and
+// those of few points, below dd's error at all lengths; what that took, as
+// multiples of dd's error:
 //   4096 points, mean 10 and noise: 1.7 with high words rounded down in every
 //     stage and a bit of the range unused, 0.8 as it is (xf_rounds, xf_excess);
 //   512 points, mean 1000 and noise, r2c: 1.6 with one bit of the range kept free
-//     for the split's sum, 0.8 with the sum halved (xf_half_sum).
+//     for the split's sum, 0.8 with the sum halved (xf_half_sum);
+//   729 points of which 8 are not zero: 2.8 without going up, 0.4 with it.
 #pragma once
 
 #include <stdint.h>
@@ -91,6 +95,9 @@ PFGB_HD xf xf_product(uint64_t p, float f) {
 // without, 891 us, 930 us with every stage rounded.  Smooth lines, up to 2048
 // points but for 2560, stay below dd's error without.
 PFGB_HD constexpr bool xf_rounds(int logm) { return logm > 10; }
+// Power-of-two lines that go up where a shift of 1 is too much: three stages lose
+// too little for it.
+PFGB_HD constexpr bool xf_ups(int logm) { return logm > 9; }
 
 // a c, in a's unit
 PFGB_HD xf operator*(xf a, xf c) {
@@ -196,6 +203,18 @@ PFGB_HD xf xf_shift(xf a, int s) {
   }
   return xf(a.h >> s, f_mul(f, f_add(a.l, xf_i2f(a.h & ((1 << s) - 1)))));
 }
+// a in units 2^u times smaller
+PFGB_HD xf xf_up(xf a, int u) {
+#if defined(__CUDA_ARCH__)
+  const float t = f_mul(a.l, __uint_as_float((unsigned)(127 + u) << 23));
+  const int i = __float2int_rn(t);
+#else
+  const float t = f_mul(a.l, (float)(1 << u));
+  const int i = (int)__builtin_rintf(t);
+#endif
+  return xf((int)((unsigned)a.h << u) + i, f_sub(t, xf_i2f(i)));
+}
+
 // Bits of a line with largest h or ~h m beyond what a butterfly of radix r <= 8
 // takes: 1.5 r m (1.5 and not sqrt 2 for the complex moduli, and for what the
 // fractions add) is to stay below 2^31.
@@ -210,6 +229,10 @@ PFGB_HD int xf_excess(unsigned m, int r) { return xf_bits(((m >> 4) + 1u) * (3u 
 // Shift of the twiddles before that butterfly, within 1 .. 3: with moduli up to
 // 0.95 2^31 three are enough.
 PFGB_HD int xf_shift_of(int excess) { return excess < 1 ? 1 : excess > kXfShifts ? kXfShifts : excess; }
+// Bits that the line's values go up by before the shift of 1: 0 unless that
+// shift would leave three free, then all of them, at most 4.  A line of zeros
+// (the rest of a last tile: far below any other) stays.
+PFGB_HD int xf_up_of(int excess) { return (unsigned)(-2 - excess) > 13u ? 0 : excess < -3 ? 4 : 1 - excess; }
 // r = 2^lr: one instruction less
 PFGB_HD int xf_excess_pow2(unsigned m, int lr) { return xf_bits(m + (m >> 1)) - 31 + lr; }
 PFGB_HD int xf_stage_shift(unsigned m, int lr) { return xf_shift_of(xf_excess_pow2(m, lr)); }

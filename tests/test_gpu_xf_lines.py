@@ -1,4 +1,5 @@
-"""Float64 lines that do not grow like noise (a dominant mean, a ramp, a tone) on the integer-float stages, power-of-two and smooth
+"""Float64 lines that do not grow like noise (a dominant mean, a ramp, a tone, few
+points among zeros) on the integer-float stages, power-of-two and smooth
 lengths, every operation of those passes.  Bound per line: the double-float
 stages' error of such lines, 1.3e-14 at most (tests/test_xf_lines.py, which
 holds the integer-float ones below it), and two conversions of 2^-50: 1.5e-14;
@@ -17,21 +18,23 @@ def _lines(n, cplx):
     """One line of each kind, along axis 0."""
     rng = np.random.default_rng(n)
     j = np.arange(n)
-    noise = rng.standard_normal((n, 5))
+    noise = rng.standard_normal((n, 7))
     if cplx:
-        noise = noise + 1j * rng.standard_normal((n, 5))
+        noise = noise + 1j * rng.standard_normal((n, 7))
     x = noise.copy()
     x[:, 0] += 10
     x[:, 1] += 1000
     x[:, 2] = j / n
     x[:, 3] += 30 * (np.exp(2j * np.pi * 3 * j / n) if cplx else np.cos(2 * np.pi * 3 * j / n))
+    x[:, 4] = np.where(j == n // 3, noise[:, 4], 0)
+    x[:, 5] = np.where(j % (n // 8 + 1) == 0, noise[:, 5], 0)
     return x
 
 
 def _apply(tr, x, permute):
     plan = P.PencilFFTPlan(x.shape, (tr, T.NoTransform()), np.float64, permute_dims=permute, extra_dims=(4,))
     u = plan.allocate_input()
-    u.copy_from_logical(np.stack([x] * 4, axis=2))  # 20 lines: the smooth-length pass from 16 complex ones on
+    u.copy_from_logical(np.stack([x] * 4, axis=2))  # 28 lines: the smooth-length pass from 16 complex ones on
     return plan, (plan * u).to_logical()
 
 

@@ -98,7 +98,8 @@ static xf_tw entry(cld w, int s) {
   memcpy(&e, t.data(), sizeof e);
   return e;
 }
-template <bool ROUND> void twiddle(C<xf>& v, cld w, int q, int sh) {
+template <bool ROUND> void twiddle(C<xf>& v, cld w, int q, int sh, int up) {
+  if (up) v = {xf_up(v.re, up), xf_up(v.im, up)};
   if (q == 0) v = {xf_shift<ROUND>(v.re, sh), xf_shift<ROUND>(v.im, sh)};
   else xf_twiddle<false, ROUND>(v.re, v.im, entry(w, sh));
 }
@@ -109,13 +110,14 @@ template <typename R> int stages(std::vector<C<R>>& x, const std::vector<int>& r
   std::vector<C<R>> y(M);
   int Ls = 1, shifts = 0;
   for (const int& r : rad) {
-    int sh = 0;
+    int sh = 0, up = 0;
     if constexpr (std::is_same<R, xf>::value) if (Ls > 1) {
       unsigned m = 0;
       for (auto& v : x) m = std::max({m, (unsigned)(v.re.h ^ (v.re.h >> 31)), (unsigned)(v.im.h ^ (v.im.h >> 31))});
       const int excess = M & (M - 1) ? xf_excess(m, r) : xf_excess_pow2(m, r == 8 ? 3 : r == 4 ? 2 : 1);
       sh = xf_shift_of(excess);
-      shifts += sh;
+      up = M & (M - 1) ? xf_up_of(excess + (r < 4)) : xf_ups(31 - __builtin_clz(M)) ? xf_up_of(excess) : 0;
+      shifts += sh - up;
     }
     for (int b = 0; b < M / r; ++b) {
       const int j = b % Ls;
@@ -125,8 +127,8 @@ template <typename R> int stages(std::vector<C<R>>& x, const std::vector<int>& r
         if (Ls == 1) continue;
         const cld w = std::polar((ld)1, -2 * PI * q * j / (r * Ls));
         if constexpr (std::is_same<R, xf>::value) {
-          if (rounds && (int)(&r - rad.data()) + 2 >= (int)rad.size()) twiddle<true>(v[q], w, q, sh);
-          else twiddle<false>(v[q], w, q, sh);
+          if (rounds && (int)(&r - rad.data()) + 2 >= (int)rad.size()) twiddle<true>(v[q], w, q, sh, up);
+          else twiddle<false>(v[q], w, q, sh, up);
         } else if (q) {
           const dd wr = split(w.real()), wi = split(w.imag());
           v[q] = {v[q].re * wr - v[q].im * wi, v[q].re * wi + v[q].im * wr};
@@ -172,8 +174,8 @@ int main(int argc, char** argv) {  // length, radices
   for (const char* q = argv[2]; *q; ++q) rad.push_back(*q - '0');
   std::mt19937_64 g(M);
   std::normal_distribution<double> un(0, 1);
-  const char* names[] = {"noise", "mean 1", "mean 10", "mean 1000", "ramp", "tone", "corner", "k^-2"};
-  for (int kind = 0; kind < 8; ++kind) {
+  const char* names[] = {"noise", "mean 1", "mean 10", "mean 1000", "ramp", "tone", "corner", "point", "two points", "eight points", "k^-2"};
+  for (int kind = 0; kind < 11; ++kind) {
     ld ex = 0, ed = 0;
     for (int rep = 0; rep < 4; ++rep) {
       std::vector<cld> x(M);
@@ -187,10 +189,13 @@ int main(int argc, char** argv) {  // length, radices
                : kind == 4 ? cld((ld)i / M, rep % 2 ? 0 : 1 - (ld)i / M)
                : kind == 5 ? n + std::polar((ld)30, t)
                : kind == 6 ? cld(1, 1) * std::polar((ld)1, PI / 2 * (i * rep % 4))
+               : kind == 7 ? (i == k0 ? n : cld(0))
+               : kind == 8 ? (i == k0 || i == (k0 * 3 + 1) % M ? n : cld(0))
+               : kind == 9 ? (i % (M / 8 + 1) == 0 ? n : cld(0))
                            : n / (ld)((1 + std::min(i, M - i)) * (1 + std::min(i, M - i)));
         x[i] *= scale;
       }
-      if (kind == 7) fft(x);
+      if (kind == 10) fft(x);
       ld mx = 0;
       for (auto& v : x) {
         v = cld((double)v.real(), (double)v.imag());
@@ -267,4 +272,4 @@ def driver(tmp_path_factory):
 def test_xf_lines_are_no_less_exact_than_double_float(driver, n):
     out = subprocess.run([str(driver), str(n), "".join(map(str, radices(n)))], check=True, capture_output=True,
                          text=True).stdout
-    assert out.count("\n") == 8 and all(line.endswith(" 1") for line in out.splitlines()), out
+    assert out.count("\n") == 11 and all(line.endswith(" 1") for line in out.splitlines()), out

@@ -37,7 +37,9 @@ static cudaError_t launch_pass_kernel(void (*kernel)(A), int64_t grid, int threa
   c.stream = s;
   c.attrs = &overlap;
   c.numAttrs = 1;
-  return cudaLaunchKernelEx(&c, kernel, args);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kernel, args);
+  if (e != cudaSuccess) cudaGetLastError();  // reported here, and not by the caller's next check
+  return e;
 }
 
 }  // namespace pfgb

@@ -386,7 +386,39 @@ __device__ __forceinline__ void stage(Cx<R>* zl, bool line_ok, int b, int Lc, in
   __syncthreads();
 }
 
-template <int SIGN, typename R>
+// The same with K butterflies a thread (b, b + threads, ...), for the one line of
+// a tile that has more of them than the block has threads: K RAD values are held
+// over the barrier, no more than the largest radix's 16 (Lc <= 8192).
+template <int RAD, int K, int SIGN, typename R>
+__device__ __forceinline__ void stage_many(Cx<R>* zl, int Lc, int Ls, const void* tw) {
+  const int T = Lc / RAD, b0 = threadIdx.x, nth = blockDim.x;
+  Cx<R> v[K][RAD];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int b = b0 + k * nth;
+    if (b >= T) break;
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) v[k][r] = zl[b + r * T];
+    if (Ls > 1) {
+      const int tstep = b % Ls * (Lc / (Ls * RAD));
+#pragma unroll
+      for (int r = 1; r < RAD; ++r) v[k][r] = v[k][r] * twid<SIGN, R>(tw, r * tstep);
+    }
+    dft_any<RAD, SIGN>(v[k], tw, Lc);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const int b = b0 + k * nth;
+    if (b >= T) break;
+    const int j = b % Ls, base = (b - j) * RAD + j;
+#pragma unroll
+    for (int r = 0; r < RAD; ++r) zl[base + r * Ls] = v[k][r];
+  }
+  __syncthreads();
+}
+
+template <int SIGN, bool MANY, typename R>
 __device__ void stockham(Cx<R>* z, const PassArgs& a, int Lc) {
   const int p = threadIdx.x / a.bpl;
   const int b = threadIdx.x % a.bpl;
@@ -395,6 +427,17 @@ __device__ void stockham(Cx<R>* z, const PassArgs& a, int Lc) {
   int Ls = 1;
   for (int s = 0; s < a.nst; ++s) {
     const int rd = a.rad[s];
+    if (MANY && Lc / rd > (int)blockDim.x) {  // one line of at most 8192 points, 1024 threads
+      switch (rd) {
+        case 2: stage_many<2, 4, SIGN, R>(zl, Lc, Ls, a.tw); break;
+        case 3: stage_many<3, 3, SIGN, R>(zl, Lc, Ls, a.tw); break;
+        case 4: stage_many<4, 2, SIGN, R>(zl, Lc, Ls, a.tw); break;
+        case 5: stage_many<5, 2, SIGN, R>(zl, Lc, Ls, a.tw); break;
+        default: stage_many<7, 2, SIGN, R>(zl, Lc, Ls, a.tw); break;  // (8192 / 8 is no more than 1024)
+      }
+      Ls *= rd;
+      continue;
+    }
     switch (rd) {
       case 2: stage<2, SIGN, R>(zl, line_ok, b, Lc, Ls, a.tw); break;
       case 3: stage<3, SIGN, R>(zl, line_ok, b, Lc, Ls, a.tw); break;
@@ -493,7 +536,10 @@ __device__ __forceinline__ Cx<R> r2r_post(const Cx<R>* zl, const PassArgs& a, in
 // ---------------------------------------------------------------------------
 // The pass kernel.
 // ---------------------------------------------------------------------------
-template <typename R>
+// MANY: lines with more butterflies in a stage than the block has threads (a
+// kernel of its own: the stages for them would add half as much again to the
+// spills of the ordinary one)
+template <typename R, bool MANY>
 __global__ void __launch_bounds__(1024) pass_kernel(const PassArgs a) {
   pass_enter();
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -593,7 +639,7 @@ __global__ void __launch_bounds__(1024) pass_kernel(const PassArgs a) {
 
   // ---- core DFT ----
   if (a.L == 0) {
-    if (a.sign < 0) stockham<-1, R>(z, a, Lc); else stockham<1, R>(z, a, Lc);
+    if (a.sign < 0) stockham<-1, MANY, R>(z, a, Lc); else stockham<1, MANY, R>(z, a, Lc);
   } else {
     const Cx<R>* chirp = reinterpret_cast<const Cx<R>*>(a.chirp);
     const Cx<R>* bf = reinterpret_cast<const Cx<R>*>(a.bfilt);
@@ -604,14 +650,14 @@ __global__ void __launch_bounds__(1024) pass_kernel(const PassArgs a) {
       zl[j] = j < a.M ? zl[j] * chirp[j] : mk(R(0), R(0));
     }
     __syncthreads();
-    stockham<-1, R>(z, a, Lc);
+    stockham<-1, MANY, R>(z, a, Lc);
     for (int e = tid; e < tot; e += nth) {
       const int p = e / Lc, j = e % Lc;
       Cx<R>* zl = z + (size_t)p * a.lp;
       zl[j] = zl[j] * bf[j];
     }
     __syncthreads();
-    stockham<1, R>(z, a, Lc);
+    stockham<1, MANY, R>(z, a, Lc);
     const int tot2 = a.clines * a.M;
     for (int e = tid; e < tot2; e += nth) {
       const int p = e / a.M, j = e % a.M;

@@ -11,20 +11,22 @@ namespace pfgb {
 
 int fail_cuda(cudaError_t e, const char* what);
 
-template <typename R>
+template <typename R, bool MANY>
 static int launch_pass_t(const PassArgs& A, int64_t grid, int threads, size_t smem, cudaStream_t s) {
   static bool configured[kMaxDevicesConfigured] = {};
-  int rc = ensure_smem_attr(pass_kernel<R>, 200 * 1024, configured, "cudaFuncSetAttribute(pass_kernel)");
+  int rc = ensure_smem_attr(pass_kernel<R, MANY>, 200 * 1024, configured, "cudaFuncSetAttribute(pass_kernel)");
   if (rc || grid == 0) return rc;
-  const cudaError_t e = launch_pass_kernel(pass_kernel<R>, grid, threads, smem, s, A);
+  const cudaError_t e = launch_pass_kernel(pass_kernel<R, MANY>, grid, threads, smem, s, A);
   if (e != cudaSuccess) return fail_cuda(e, "pass_kernel launch");
   return PFGB_OK;
 }
 
 int launch_pass(int real_bytes, const PassArgs& A, int64_t grid, int threads, size_t smem,
                 cudaStream_t s) {
-  if (real_bytes == 8) return launch_pass_t<double>(A, grid, threads, smem, s);
-  return launch_pass_t<float>(A, grid, threads, smem, s);
+  // (Float32 lines beyond the convolution's length go through a split)
+  if (real_bytes == 8 && A.bpl > 1024) return launch_pass_t<double, true>(A, grid, threads, smem, s);
+  if (real_bytes == 8) return launch_pass_t<double, false>(A, grid, threads, smem, s);
+  return launch_pass_t<float, false>(A, grid, threads, smem, s);
 }
 
 int launch_copy(int elt_bytes, const CopyArgs& C, cudaStream_t s) {

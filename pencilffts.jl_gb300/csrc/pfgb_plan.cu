@@ -644,12 +644,9 @@ static int upload_tc_table(pfgb_plan* P, int logm, int sign, const void** out) {
   return PFGB_OK;
 }
 
-// Radix plan for a DFT length of the generic kernel: returns false if a prime
-// factor > 13 remains, or if a stage has more butterflies than a block has
-// threads (the stages run in place, one butterfly a thread).
-constexpr int kMaxButterflies = 1024;
-static bool factor_radices(int n, std::vector<int>& rad) {
-  const int len = n;
+// Radices of a DFT length of the generic kernel: returns false if a prime factor
+// > 13 remains.
+static bool radices_of(int n, std::vector<int>& rad) {
   rad.clear();
   int e = 0;
   while (n % 2 == 0) { n /= 2; ++e; }
@@ -666,7 +663,13 @@ static bool factor_radices(int n, std::vector<int>& rad) {
     }
   }
   for (int p : odds) rad.push_back(p);
-  return rad.empty() || len / *std::min_element(rad.begin(), rad.end()) <= kMaxButterflies;
+  return true;
+}
+// The same with at most one butterfly a thread of a block in each stage, which
+// the lengths go by that have another form (a convolution, a split).
+constexpr int kMaxButterflies = 1024;
+static bool factor_radices(int n, std::vector<int>& rad) {
+  return radices_of(n, rad) && (rad.empty() || n / *std::min_element(rad.begin(), rad.end()) <= kMaxButterflies);
 }
 
 // ---------------------------------------------------------------------------
@@ -679,9 +682,13 @@ static int prepare_core(pfgb_plan* P, Pass& ps, int M) {
   if (!factor_radices(M, rad)) {
     int L = 1;
     while (L < 2 * M - 1) L <<= 1;
-    ps.L = L;
-    Lc = L;
-    factor_radices(L, rad);
+    // a convolution beyond the core: several butterflies a thread, where the
+    // length has radices (native Float64; the other plans split such lines)
+    if (L <= kMaxLc || M > kMaxLc || P->rb != 8 || !radices_of(M, rad)) {
+      ps.L = L;
+      Lc = L;
+      radices_of(L, rad);
+    }
   }
   if (Lc > kMaxLc)
     return fail(PFGB_ERR_UNSUPPORTED, "transform length " + std::to_string(M) +
@@ -3160,6 +3167,7 @@ static int plan_build(const pfgb_plan_desc* desc, pfgb_plan** out, bool query_on
         } else {
           PassArgs A;
           std::memset(&A, 0, sizeof(A));
+          A.bpl = ps.bpl;
           rc = launch_pass(P->rb, A, 0, 0, 0, nullptr);
         }
       }

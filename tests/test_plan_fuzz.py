@@ -66,3 +66,15 @@ def test_any_length_plans():
     for n in (8209, 65537):
         P.plan_query((n,), T.RFFT(), np.float32)
         P.plan_query((n,), T.R2R(T.REDFT01), np.float64)
+
+
+@pytest.mark.parametrize("precision", ["default", "native", "fx"])
+def test_smooth_lengths_of_the_generic_core_plan(precision):
+    """Lengths up to 8192 points without a prime factor above 13 plan at every
+    Float64 precision, also where the smallest radix leaves more butterflies
+    than a block has threads and the convolution form would be too long."""
+    for n in (4096, 4374, 4719, 6006, 6561, 7203, 8100, 8190, 8192):
+        for tr in (T.FFT(), T.RFFT(), T.R2R(T.DHT)):
+            P.plan_query((n, 3), (tr, T.NoTransform()), np.float64, precision=precision)
+        if n % 2 == 0:
+            P.plan_query((n // 2, 3), (T.R2R(T.REDFT01), T.NoTransform()), np.float64, precision=precision)

@@ -1179,12 +1179,19 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
   if (ps.smem > 200 * 1024)
     return fail(PFGB_ERR_UNSUPPORTED, "line does not fit in shared memory");
   ps.zero_fill = ps.L > 0 || (ps.op == OP_R2R_C || ps.op == OP_R2R_R);
+  auto keep_generic = [&ps] {  // the generic kernel's geometry, where it is an alternative
+    ps.g_lines = ps.lines;
+    ps.g_clines = ps.clines;
+    ps.g_threads = ps.threads;
+    ps.g_smem = ps.smem;
+  };
   // other c2c / r2c / c2r lines of 2, 3, 5 and 7 only take the smooth-length
   // pass (integer-float for Float64 data unless native FP64 was requested;
   // Float64 lines above 2048 points stay in FP64, which is more precise)
   if ((ps.op == OP_C2C || ps.op == OP_R2C || ps.op == OP_C2R) &&
       !(P->rb == 8 && (P->precision == PFGB_PRECISION_NATIVE || M > 2048))) {
     bool smooth = false;
+    if (M <= 2048) keep_generic();
     rc = sm_form(P, ps, M > 2048, smooth);
     if (rc || smooth) return rc;
   }
@@ -1192,10 +1199,7 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
   // pass (double-float for Float64 data unless native FP64 was requested)
   if ((ps.op == OP_C2C || ps.op == OP_R2C || ps.op == OP_C2R) && M >= 2 && M <= 2048 &&
       !(P->rb == 8 && P->precision == PFGB_PRECISION_NATIVE)) {
-    ps.g_lines = ps.lines;
-    ps.g_clines = ps.clines;
-    ps.g_threads = ps.threads;
-    ps.g_smem = ps.smem;
+    keep_generic();
     return bluestein_form(P, ps);
   }
   return PFGB_OK;
@@ -1626,7 +1630,7 @@ static int launch_bs(const pfgb_plan* P, const Pass& ps, const FastArgs& F, int6
 // The generic-kernel form of a Bluestein pass (its own geometry)
 static Pass generic_form(const Pass& ps) {
   Pass g = ps;
-  g.bs = false;
+  g.bs = g.sm = false;
   g.lines = ps.g_lines;
   g.clines = ps.g_clines;
   g.threads = ps.g_threads;
@@ -2350,7 +2354,7 @@ static int execute(pfgb_plan* P, const Direction& dir, void* dst, const void* sr
         rc = launch_plain(P, ps, F, grid, s);
       }
       if (rc) return rc;
-    } else if (ps.mr || ps.sm) {
+    } else if (ps.mr || (ps.sm && ps.variant != 2)) {
       FastArgs F;
       int64_t grid = 0;
       int rc = make_fast_args(P, ps, in, out, normalise && i == last_tr, F, grid, i == dpass ? dv : nullptr);
@@ -2372,7 +2376,7 @@ static int execute(pfgb_plan* P, const Direction& dir, void* dst, const void* sr
       // generic kernel (a Bluestein-eligible pass runs here with its generic
       // geometry when a fused sum of derivatives applies to it, or when the
       // planner measured this form faster)
-      const Pass g = ps.bs ? generic_form(ps) : ps;
+      const Pass g = ps.bs || ps.sm ? generic_form(ps) : ps;
       PassArgs A;
       int64_t grid = 0;
       int rc = make_args(P, g, in, out, normalise && i == last_tr, A, grid, i == dpass ? dv : nullptr);
@@ -3155,6 +3159,11 @@ static int plan_build(const pfgb_plan_desc* desc, pfgb_plan** out, bool query_on
           FastArgs F;
           std::memset(&F, 0, sizeof(F));
           rc = launch_sm(P, ps, F, 0, nullptr);
+          if (!rc && ps.g_threads > 0) {
+            PassArgs A;
+            std::memset(&A, 0, sizeof(A));
+            rc = launch_pass(P->rb, A, 0, 0, 0, nullptr);
+          }
         } else if (ps.bs) {
           FastArgs F;
           std::memset(&F, 0, sizeof(F));
@@ -3242,9 +3251,9 @@ int pfgb_plan_set_timing(pfgb_plan* P, int on) {
 // buffers filled with normal numbers (bytes 0x3F), and the faster is kept.
 // Alternatives today: c2r passes of Float32 and double-float plans, plain
 // fast_pass or the TMA-fed persistent form (when the buffers satisfy its
-// alignment); lines taken by the Bluestein register pass, that pass or the
-// generic kernel (radix 2..16 stages in shared memory, or its own Bluestein
-// for long lines).
+// alignment); lines up to 2048 points taken by the Bluestein register pass or
+// the smooth-length pass, that pass or the generic kernel (radix 2..16 stages
+// in shared memory, or its own Bluestein for long lines).
 static int autotune_passes(pfgb_plan* P) {
   const int e1023 = 1023;
   for (auto* dir : {&P->fwd, &P->bwd}) {
@@ -3303,12 +3312,12 @@ static int autotune_passes(pfgb_plan* P) {
       if (rc) return rc;
     }
   }
-  // Bluestein-eligible passes: the Bluestein register pass (variant -1)
-  // against the generic kernel (variant 2) on the same buffers
+  // Bluestein register or smooth-length pass (variant -1) against the generic
+  // kernel (variant 2) on the same buffers
   for (auto* dir : {&P->fwd, &P->bwd}) {
     for (auto& ps : dir->passes) {
-      if (!ps.bs) continue;
-      const std::string wkey = wisdom_key(P, ps, "bluestein-generic");
+      if (!ps.bs && !(ps.sm && ps.g_threads > 0)) continue;
+      const std::string wkey = wisdom_key(P, ps, ps.sm ? "smooth-generic" : "bluestein-generic");
       int wv = 0;
       if (wisdom_lookup(wkey, &wv)) {
         ps.variant = wv;
@@ -3340,7 +3349,7 @@ static int autotune_passes(pfgb_plan* P) {
             F.bs_chirp = ps.bs_chirp;
             F.bs_filt = ps.bs_filt;
             F.div_m = make_div31(ps.op == OP_R2C ? ps.M / 2 + 1 : ps.M);
-            if (!rc) rc = launch_bs(P, ps, F, grid, 0);
+            if (!rc) rc = ps.sm ? launch_sm(P, ps, F, grid, 0) : launch_bs(P, ps, F, grid, 0);
           } else {
             const Pass g = generic_form(ps);
             PassArgs A;
@@ -3458,7 +3467,7 @@ int pfgb_plan_get_timing(pfgb_plan* P, pfgb_pass_timing* out, int max, int* n) {
                         : ps.variant == 1 ? (P->rb == 8 ? "fast_pass_tma<dd>" : "fast_pass_tma<float>")
                         : ps.fast ? (P->rb == 4 ? "fast_pass<float>" : P->fx ? "fast_pass<fx>" : "fast_pass<dd>")
                         : ps.mr ? (P->rb == 4 ? "mr_pass<float>" : "mr_pass<dd>")
-                        : ps.sm ? (P->rb == 4 ? "sm_pass<float>" : "sm_pass<dd>")
+                        : ps.sm && ps.variant != 2 ? (P->rb == 4 ? "sm_pass<float>" : "sm_pass<dd>")
                         : ps.bs && ps.variant != 2 ? (P->rb == 4 ? "bs_pass<float>" : "bs_pass<dd>")
                                   : (P->rb == 8 ? "pass_kernel<double>" : "pass_kernel<float>");
     std::snprintf(e.kernel, sizeof(e.kernel), "%s", kname);

@@ -57,3 +57,43 @@ def test_wisdom_reused_by_measured_plans(cuda, tmp_path):
     check_plan(plan2, seed=3)
     check_plan(plan, seed=3)
     P.forget_wisdom()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("real", [np.float64, np.float32])
+def test_smooth_lines_are_measured(cuda, real):
+    """Lines of 100 points: the smooth-length pass against the generic kernel, in
+    both directions; a plan that takes either from wisdom has the oracle's results."""
+    from helpers import T
+    from test_gpu_parity import check_plan
+    P.forget_wisdom()
+    dims = (100, 64, 40)
+    plan = P.PencilFFTPlan(dims, T.RFFT(), real, fftw_flags=P.FFTW_MEASURE)
+    entries, hits = P.wisdom_stats()
+    assert entries >= 2 and hits == 0
+    check_plan(plan, seed=4)
+    P.forget_wisdom()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("choice", [-1, 2])
+def test_measured_choice_of_smooth_lines_is_taken(cuda, tmp_path, choice):
+    from helpers import T
+    from test_gpu_parity import check_plan
+    P.forget_wisdom()
+    dims = (45, 64, 40)
+    P.PencilFFTPlan(dims, T.RFFT(), np.float64, fftw_flags=P.FFTW_MEASURE)
+    f = tmp_path / "w.wisdom"
+    P.export_wisdom(f)
+    head, *lines = f.read_text().splitlines()
+    lines = [f"{choice}\t" + x.split("\t")[1] if "smooth-generic" in x else x for x in lines]
+    f.write_text("\n".join([head] + lines) + "\n")
+    P.forget_wisdom()
+    P.import_wisdom(f)
+    plan = P.PencilFFTPlan(dims, T.RFFT(), np.float64, fftw_flags=P.FFTW_MEASURE)
+    check_plan(plan, seed=5)
+    plan.set_timing(True)
+    plan.ldiv(plan * plan.allocate_input())
+    kernels = {e["kernel"] for e in plan.get_timing()}
+    assert ("pass_kernel<double>" if choice == 2 else "sm_pass<dd>") in kernels
+    P.forget_wisdom()

@@ -764,7 +764,7 @@ static int tile_dim(const Pass& ps);
 // with the square root of the radices from it on, and with 8 8 8 5 such a line
 // with a large mean had 1.4 times the error of the double-float form (8 8 5 4 2:
 // 0.95).
-static bool sm_radices(int M, bool f64, int& nst, int (&r)[kSmStages]) {
+static bool sm_radices(int M, bool f64, int& nst, int (&r)[kSmStages], int most = 16) {
   if (f64 && M > 2048 && M % 8 == 0) {
     if (!sm_radices(M / 8, f64, nst, r) || nst > kSmStages - 2) return false;
     r[nst++] = 4;
@@ -784,7 +784,7 @@ static bool sm_radices(int M, bool f64, int& nst, int (&r)[kSmStages]) {
     }
     if (depth >= kSmStages || depth >= best_n) return;
     for (int i = from; i < (int)(sizeof(all) / sizeof(all[0])); ++i) {
-      if (f64 && all[i] > 8) continue;
+      if (all[i] > (f64 ? 8 : most)) continue;
       if (m % all[i]) continue;
       cur[depth] = all[i];
       self(self, m / all[i], depth + 1, i, sum + all[i]);
@@ -831,8 +831,13 @@ static int sm_best_pitch(int M, int w, int q, int r0, int ebytes) {
 // (3 or 5 times a power of two; its Float32 form stays the faster one: 384^3
 // 0.86 ms, where 360^3 takes 0.83 here), with 16 complex lines or more.  Fewer
 // lines keep the Bluestein or mixed-radix tile where those have the length
-// (few): launch latency sets their time, and the plans that ask for those
-// kernels by name in tests have few lines.  Measured round trips, Bluestein or
+// (few).  Forward + inverse of 1 to 15 lines in a graph, Bluestein against this
+// pass, us: Float32 100 points 7.5 and 13.0, 360 9.4 and 10.4, 1000 10.6 and
+// 14.0; Float64 100 points 14.4 to 17.4 and 15.6, 360 20.0 and 16.3, 1000 22.5
+// and 19.4, 2000 35.8 and 26.0.  So the line is right for Float32; Float64 lines
+// of 200 points and more would gain at any count, which is open
+// (tests/test_gpu_smooth.py asks for the Bluestein tile at 15 lines of 100).
+// Measured round trips, Bluestein or
 // (*) mixed-radix tile against this one: Float64 RFFT 100^3 0.213 -> 0.082 ms,
 // 240^3 1.98 -> 0.64, 360^3 9.73 -> 2.42, *384^3 3.97 -> 2.36, FFT *96^3 0.286
 // -> 0.100, *24^3 0.139 -> 0.045, 1000^2 0.260 -> 0.124; Float32 RFFT 360^3 3.45 -> 0.83, 120^3 0.088 -> 0.069,
@@ -855,6 +860,17 @@ static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
   for (int d = 0; d < ps.lin.D; ++d)
     if (d != ps.axis && d != td) outer *= ps.lin.size[d];
   if (ncl * outer < 16 && !few) return PFGB_OK;
+  // Few Float32 points on lines along the memory wait for one tile's loads and
+  // instructions: radices up to 8 (forward + inverse of 16 to 200 lines in a
+  // graph, us: 100 points 12.8 -> 9.8, 144 14.2 -> 9.1, 1000 (16, 48) 14.0 -> 10.9,
+  // 360 10.3 -> 10.6; 100x100 r2c plan 22.2 -> 19; Bluestein 7.6, 8.6, 10.6, 9.5)
+  if (!f64 && ps.lin.perm[0] == ps.axis && ncl * outer * M <= (1 << 17)) {
+    int n8 = 0, r8[kSmStages];
+    if (sm_radices(M, f64, n8, r8, 8)) {
+      nst = n8;
+      std::copy(r8, r8 + n8, r);
+    }
+  }
   const bool strided = ps.lin.perm[0] != ps.axis || ps.lout.perm[0] != ps.axis;
   const int ebytes = f64 ? 16 : 8, pitch = M + 1 + 128 / ebytes;  // the widest sm_best_pitch gives
   double best = 1e30;
@@ -890,7 +906,8 @@ static int sm_form(pfgb_plan* P, Pass& ps, bool few, bool& taken) {
     }
   }
   if (!tw) return PFGB_OK;
-  const std::string key = (f64 ? "smx" : "smf") + std::to_string(M);
+  std::string key = f64 ? "smx" : "smf";
+  for (int s = 0, left = M; s < nst; left /= r[s], ++s) key += std::to_string(left) + "/";
   if (!P->query_only && !P->tables.count(key)) {
     std::vector<std::complex<ld>> w;
     for (int s = 1, Ls = r[0]; s < nst; Ls *= r[s], ++s)

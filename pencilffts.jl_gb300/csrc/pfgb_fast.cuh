@@ -542,7 +542,7 @@ __device__ __forceinline__ void stages_core(Cx<R> (&v)[P], Cx<R>* z, int p, int 
         const int lr = s + 1 < SP ? 3 : REM;
         sh = xf_stage_shift(lmax, lr);
         shifts += sh;
-        if (const int up = xf_ups(LOGM) ? xf_up_of(xf_excess_pow2(lmax, lr)) : 0) {  // in place: no other thread reads this one's inputs
+        if (const int up = xf_up_of(xf_excess_pow2(lmax, lr), xf_slack(1 << lr))) {  // in place: no other thread reads this one's inputs
 #pragma unroll 1
           for (int r = 0; r < P; ++r) {
             Cx<R>& x = z[zr + padded<R, LOGM>(r * T)];
@@ -665,7 +665,12 @@ __host__ __device__ constexpr int fast_min_blocks(int logm, int op, int iom) {
                                2048 / fast_threads<R>(logm, op)
                            ? (op == OP_C2R && PFGB_FAST_F32_MINBLOCKS > 3 ? 3 : PFGB_FAST_F32_MINBLOCKS)
                            : 2048 / fast_threads<R>(logm, op)))
-         : fast_threads<R>(logm, op) >= 512 ? 2
+         : fast_threads<R>(logm, op) >= 512
+             // all forms, spills of up to 0.25 KB included (round trips with one block
+             // an SM and two: REDFT10 / 01 4096^2 885 and 745 us, DHT 869 and 680, complex
+             // lines 1376 and 1097, REDFT00 2049^2 300 and 243, REDFT11 2048^2 325 and 269,
+             // fx c2c 4096^2 1476 and 1150, divergence 64x32x4096 291 and 256)
+             ? 2
          : (fast_d23(op) || fast_d4(op)) ? 3  // two loads a position (D3) or two real lines (D2R / D3R): ~0.2-0.5 KB of spill at 64 registers
          : PFGB_FAST_DD_MINBLOCKS <= 0 ? 512 / fast_threads<R>(logm, op)
          : (op == OP_C2R && !(iom & 1) && PFGB_FAST_DD_MINBLOCKS > 4) ? 4

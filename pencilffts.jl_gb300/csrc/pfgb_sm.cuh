@@ -7,14 +7,18 @@
 // two shared-memory buffers.  A thread owns one line of the tile (p = thread
 // mod TW) and every K-th butterfly of each stage: its loads, twiddles and
 // stores need no division, its line's scale is its own, and the pitch leaves the
-// fewest bank conflicts for the tile's width (sm_best_pitch).  Radices up to 16 (Float32) or 8 (Float64, whose range bound
-// is a growth of 8 per stage) leave two or three stages for most lengths.
+// fewest bank conflicts for the tile's width (sm_best_pitch).  Radices up to 16
+// (Float32) or 8 (Float64, whose range bound is a growth of 8 per stage) leave
+// two to four stages for most lengths.
 //
 // Bound by issue slots (125 to 155 instructions a point in Float32, half of
 // them integer, before addresses were stepped in bytes) and the shared-memory
 // pipe together: 360^3 Float32 round trip 930 -> 834 us, Float64 2514 -> 2421 us
 // with byte steps, walks of their own for lanes across the lines, and the
-// pitch.
+// pitch.  Float64: 330 to 450 instructions a point at 24 warps an SM (80
+// registers).  A derivative on the input or output multiplies in FP64 (in1k),
+// whose unit then bounds the pass: 329 us for the first pass of a 240^3
+// divergence, where a pass without takes 107.
 //
 // Against the Bluestein tile, which takes these lengths through two
 // power-of-two transforms of at least twice the length: see sm_form in
@@ -265,7 +269,7 @@ __device__ __forceinline__ void sm_stage(const FastArgs& a, int s, SmThread& t, 
 }
 // The inputs of the thread's butterflies go up by some bits (xf_up), in place:
 // no other thread reads them.  Out of the stage's loop, where the branch costs more
-// (240^3 Float64 round trip 646 us; here 639; nowhere 630).
+// (240^3 Float64 round trip 646 us; here 637; nowhere 630).
 __device__ __forceinline__ void sm_up(Cx<xf>* z, const SmThread& t, int T, int M, int up) {
 #pragma unroll 1
   for (int b = t.b0; b < T; b += t.k)
@@ -563,9 +567,7 @@ __global__ void __launch_bounds__(kSmThreads, std::is_same<R, xf>::value ? 3 : 4
       const int r = a.sm_r[s], excess = xf_excess(lm[s][t.p], r) + head;
       t.sh = xf_shift_of(excess);
       shifts += t.sh;
-      // (radices of 2 and 3 may leave a bit more: noise does at 243 points, and
-      // going up each time makes 243^3 1.73 ms instead of 1.57)
-      if (const int up = xf_up_of(excess + (r < 4))) {
+      if (const int up = xf_up_of(excess, xf_slack(r))) {
         sm_up(z + za + t.p * pitch, t, M / r, M, up);
         shifts -= up;
       }

@@ -21,8 +21,8 @@
 // s = 1 (few non-zero points, small radices) goes up by some bits first
 // (xf_up_of).
 //
-// Cost: 512^3 Float64 round trip 4.14 ms with dd stages, 3.28 ms with these;
-// 256^3 complex 0.945 and 0.725 ms.
+// Cost: 512^3 Float64 round trip 4.14 ms with dd stages, 3.30 ms with these;
+// 256^3 complex 0.945 and 0.757 ms.
 //
 // Precision: each operation rounds the fraction at about 2^-24 unit, whatever the
 // value, where a dd stage's error follows the single value.  Lines of noise have
@@ -35,7 +35,13 @@
 //     stage and a bit of the range unused, 0.8 as it is (xf_rounds, xf_excess);
 //   512 points, mean 1000 and noise, r2c: 1.6 with one bit of the range kept free
 //     for the split's sum, 0.8 with the sum halved (xf_half_sum);
-//   729 points of which 8 are not zero: 2.8 without going up, 0.4 with it.
+//   729 points of which 8 are not zero: 2.8 without going up, 0.5 with it.
+// What dd does better is the line of one large value among small ones, such as the
+// spectrum of a field with a mean: its transform does not grow, so a unit of the
+// large value's 2^-27 is all there is, and the error is up to 0.63 sqrt(M) 2^-50 of
+// the line (2.5 times dd's at 512 points, 5 times at 4096; 5.6 and 11 without going
+// up).  A round trip of such a field stays below dd's error at 512^3 (mean 10 and unit
+// noise 1.6e-14 against 2.8e-14), 1.4 times above it at 4096^2 (3.6e-14 against 2.6e-14).
 #pragma once
 
 #include <stdint.h>
@@ -95,9 +101,12 @@ PFGB_HD xf xf_product(uint64_t p, float f) {
 // without, 891 us, 930 us with every stage rounded.  Smooth lines, up to 2048
 // points but for 2560, stay below dd's error without.
 PFGB_HD constexpr bool xf_rounds(int logm) { return logm > 10; }
-// Power-of-two lines that go up where a shift of 1 is too much: three stages lose
-// too little for it.
-PFGB_HD constexpr bool xf_ups(int logm) { return logm > 9; }
+// Slack of a stage of radix r (xf_up_of).  Lines of noise never come to 0 before
+// a radix of 7 or 8, so a line that does is one that the sums do not grow (the
+// spectrum of a field with a mean: its error is halved); before the smaller ones
+// they do, and going up each time costs (243^3 Float64 1.73 ms instead of 1.57 with
+// 2 for radix 3).
+PFGB_HD constexpr int xf_slack(int r) { return r > 6 ? 0 : r > 3 ? 2 : 3; }
 
 // a c, in a's unit
 PFGB_HD xf operator*(xf a, xf c) {
@@ -230,9 +239,11 @@ PFGB_HD int xf_excess(unsigned m, int r) { return xf_bits(((m >> 4) + 1u) * (3u 
 // 0.95 2^31 three are enough.
 PFGB_HD int xf_shift_of(int excess) { return excess < 1 ? 1 : excess > kXfShifts ? kXfShifts : excess; }
 // Bits that the line's values go up by before the shift of 1: 0 unless that
-// shift would leave three free, then all of them, at most 4.  A line of zeros
-// (the rest of a last tile: far below any other) stays.
-PFGB_HD int xf_up_of(int excess) { return (unsigned)(-2 - excess) > 13u ? 0 : excess < -3 ? 4 : 1 - excess; }
+// shift would leave slack + 1 bits free, then all of them, at most 4.  A line of
+// zeros (the rest of a last tile: far below any other) stays.
+PFGB_HD int xf_up_of(int excess, int slack) {
+  return (unsigned)(-slack - excess) > 13u ? 0 : excess < -3 ? 4 : 1 - excess;
+}
 // r = 2^lr: one instruction less
 PFGB_HD int xf_excess_pow2(unsigned m, int lr) { return xf_bits(m + (m >> 1)) - 31 + lr; }
 PFGB_HD int xf_stage_shift(unsigned m, int lr) { return xf_shift_of(xf_excess_pow2(m, lr)); }

@@ -3,7 +3,8 @@ points among zeros) on the integer-float stages, power-of-two and smooth
 lengths, every operation of those passes.  Bound per line: the double-float
 stages' error of such lines, 1.3e-14 at most (tests/test_xf_lines.py, which
 holds the integer-float ones below it), and two conversions of 2^-50: 1.5e-14;
-R2R lines have twiddles at their ends as well: 2e-14."""
+R2R lines have twiddles at their ends as well: 2e-14.  Spectra of fields with a
+mean, power-of-two lines: sqrt(n) 2^-50 and the conversions."""
 import numpy as np
 import pytest
 
@@ -59,6 +60,19 @@ def test_xf_lines_that_do_not_grow_like_noise(cuda, n):
         S = plan.allocate_output()
         S.copy_from_logical(np.stack([np.repeat(s, 2, axis=1)] * 4, axis=2))
         _check(plan.ldiv(S).to_logical(), np.repeat(np.fft.irfft(s, n, axis=0), 2, axis=1), 1.5e-14, "c2r")
+
+
+@pytest.mark.parametrize("n", [64, 256, 512, 1024, 4096])
+def test_xf_spectra_of_fields_with_a_mean(cuda, n):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((n, 12)) + np.repeat([10.0, 1000.0, 0.5], 4)
+    x[:, 8:] = rng.random((n, 4))
+    for tr in (T.FFT(), T.RFFT()):
+        f = x.astype(complex) if isinstance(tr, T.FFT) else x
+        plan = P.PencilFFTPlan(x.shape, (tr, T.NoTransform()), np.float64)
+        S = plan.allocate_output()
+        S.copy_from_logical(np.fft.fft(f, axis=0) if isinstance(tr, T.FFT) else np.fft.rfft(f, axis=0))
+        _check(plan.ldiv(S).to_logical()[:, :, None].repeat(4, axis=2), f, (n ** 0.5 + 2) * 2.0 ** -50, tr)
 
 
 @pytest.mark.parametrize("kind,n", [(T.REDFT10, 729), (T.RODFT10, 1000), (T.REDFT01, 729), (T.DHT, 1215), (T.REDFT00, 730),

@@ -6,7 +6,14 @@ A double-float value keeps 48 bits of itself, an integer-float one a fraction of
 the unit its whole line shares, so a dominant mean, a ramp or a few points among
 zeros are where the second could lose.  Required: per kind of line, a relative
 L2 error against long double no larger than that of the double-float stages on
-the same lines (their rms over four lines a kind)."""
+the same lines (their rms over four lines a kind).
+
+The spectrum of a field with a mean is one large value among small ones, and its
+transform does not grow.  Its unit is the large value's 2^-26 to 2^-27, and a stage's
+roundings (four of 2^-25 unit a value, 2^-50 of the large value together) add up
+over the values that an output sums: M 2^-102 from the input, M/8 2^-100 (1 + 1/8 +
+...) from the radix-8 stages, 0.63 sqrt(M) 2^-50 in all; double-float has about
+2^-47.  Required of the power-of-two lines: sqrt(M) 2^-50."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -116,7 +123,7 @@ template <typename R> int stages(std::vector<C<R>>& x, const std::vector<int>& r
       for (auto& v : x) m = std::max({m, (unsigned)(v.re.h ^ (v.re.h >> 31)), (unsigned)(v.im.h ^ (v.im.h >> 31))});
       const int excess = M & (M - 1) ? xf_excess(m, r) : xf_excess_pow2(m, r == 8 ? 3 : r == 4 ? 2 : 1);
       sh = xf_shift_of(excess);
-      up = M & (M - 1) ? xf_up_of(excess + (r < 4)) : xf_ups(31 - __builtin_clz(M)) ? xf_up_of(excess) : 0;
+      up = xf_up_of(excess, xf_slack(r));
       shifts += sh - up;
     }
     for (int b = 0; b < M / r; ++b) {
@@ -174,8 +181,9 @@ int main(int argc, char** argv) {  // length, radices
   for (const char* q = argv[2]; *q; ++q) rad.push_back(*q - '0');
   std::mt19937_64 g(M);
   std::normal_distribution<double> un(0, 1);
-  const char* names[] = {"noise", "mean 1", "mean 10", "mean 1000", "ramp", "tone", "corner", "point", "two points", "eight points", "k^-2"};
-  for (int kind = 0; kind < 11; ++kind) {
+  const char* names[] = {"noise", "mean 1", "mean 10", "mean 1000", "ramp", "tone", "corner", "point", "two points", "eight points", "k^-2",
+                         "spectrum 10", "spectrum 1000", "spectrum uniform"};
+  for (int kind = 0; kind < 14; ++kind) {
     ld ex = 0, ed = 0;
     for (int rep = 0; rep < 4; ++rep) {
       std::vector<cld> x(M);
@@ -192,10 +200,13 @@ int main(int argc, char** argv) {  // length, radices
                : kind == 7 ? (i == k0 ? n : cld(0))
                : kind == 8 ? (i == k0 || i == (k0 * 3 + 1) % M ? n : cld(0))
                : kind == 9 ? (i % (M / 8 + 1) == 0 ? n : cld(0))
+               : kind == 11 ? n + (ld)10
+               : kind == 12 ? n + (ld)1000
+               : kind == 13 ? cld((ld)(g() >> 11) * 0x1p-53L)
                            : n / (ld)((1 + std::min(i, M - i)) * (1 + std::min(i, M - i)));
         x[i] *= scale;
       }
-      if (kind == 10) fft(x);
+      if (kind >= 10) fft(x);
       ld mx = 0;
       for (auto& v : x) {
         v = cld((double)v.real(), (double)v.imag());
@@ -272,4 +283,13 @@ def driver(tmp_path_factory):
 def test_xf_lines_are_no_less_exact_than_double_float(driver, n):
     out = subprocess.run([str(driver), str(n), "".join(map(str, radices(n)))], check=True, capture_output=True,
                          text=True).stdout
-    assert out.count("\n") == 11 and all(line.endswith(" 1") for line in out.splitlines()), out
+    lines = out.splitlines()
+    assert len(lines) == 14 and all(line.endswith(" 1") for line in lines[:11]), out
+
+
+@pytest.mark.parametrize("n", [64, 128, 256, 512, 1024, 2048, 4096])
+def test_xf_lines_of_one_large_value(driver, n):
+    out = subprocess.run([str(driver), str(n), "".join(map(str, radices(n)))], check=True, capture_output=True,
+                         text=True).stdout
+    errors = [float(line.split()[-3]) for line in out.splitlines()[11:]]
+    assert len(errors) == 3 and max(errors) <= n ** 0.5 * 2.0 ** -50, out

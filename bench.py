@@ -65,7 +65,7 @@ def workload(args):
 
 
 ARITHMETIC = {
-    ("f64", "default"): "dd (2xFP32, 48-bit significand) for power-of-two lines",
+    ("f64", "default"): "int32 + FP32 pairs in the butterflies, dd (2xFP32, 48-bit significand) around them",
     ("f64", "native"): "FP64",
     ("f64", "fx"): "block floating point (int64 components, per-line exponent)",
     ("f32", "default"): "FP32",

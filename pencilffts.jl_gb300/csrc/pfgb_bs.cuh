@@ -1,6 +1,6 @@
 // Bluestein (chirp-z) register pass: lines of any length M <= 2048 for c2c,
-// r2c and c2r, in FP32 or in double-float (doubles in and out, one exponent
-// per complex line), any input / output layout; c2c lines take the fused
+// r2c and c2r, in FP32 or (Float64 data) in double-float around integer-float
+// register stages (doubles in and out, one exponent per complex line), any input / output layout; c2c lines take the fused
 // spectral derivative (i k times the input or the output).
 //
 // With w[j] = exp(s i pi j^2 / M) (s the transform's sign),

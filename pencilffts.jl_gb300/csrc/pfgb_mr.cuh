@@ -7,17 +7,19 @@
 // Phase A: thread (line p, index b) holds the positions n1 = b + r N/8
 // (r < 8) of its line; for each r it loads the R0 inputs x[n1 + N n2],
 // computes their R0-point DFT in registers (symmetric split; roots of unity
-// from the M-point table), multiplies by the twiddles W_M^(n1 k2) and parks
-// value k2 in sub-line k2 of shared memory.  Phase B: each sub-line is an
+// from the first R0 entries of tw2), multiplies by the twiddles W_M^(n1 k2)
+// (its other entries, consecutive for consecutive n1) and parks value k2 in
+// sub-line k2 of shared memory.  Phase B: each sub-line is an
 // N-point transform computed by the power-of-two register stages
 // (fast_stages), its outputs X[k2 + R0 k1] left in the sub-line at k1.
 // Store: one loop over the tile's outputs through shared memory (c2c, the
 // r2c split of two packed real lines, or the two real outputs of a c2r
 // line), coalesced along the output's contiguous dimension.
 //
-// Float64 data compute in double-float (dd) with one power-of-two scale per
-// complex line (its largest input exponent), doubles in and out; Float32 in
-// FP32.
+// Float64 data compute phase A in double-float (dd) and phase B in integer-float
+// pairs (fast_stages), with one power-of-two scale per complex line (its largest
+// input exponent), doubles in and out; Float32 in FP32.  Float64 lines come here
+// in plans of fewer than 16 complex lines; the others take sm_pass.
 #pragma once
 
 #include "pfgb_fast.cuh"

@@ -763,7 +763,7 @@ static int tile_dim(const Pass& ps);
 // points (2560 is the one) ends in radices of 4 and 2: a stage's roundings grow
 // with the square root of the radices from it on, and with 8 8 8 5 such a line
 // with a large mean had 1.4 times the error of the double-float form (8 8 5 4 2:
-// 0.95).
+// 0.85).
 static bool sm_radices(int M, bool f64, int& nst, int (&r)[kSmStages], int most = 16) {
   if (f64 && M > 2048 && M % 8 == 0) {
     if (!sm_radices(M / 8, f64, nst, r) || nst > kSmStages - 2) return false;
@@ -1213,7 +1213,7 @@ static int prepare_pass(pfgb_plan* P, Pass& ps) {
     if (rc || smooth) return rc;
   }
   // other c2c / r2c / c2r lines up to 2048 points take the Bluestein register
-  // pass (double-float for Float64 data unless native FP64 was requested)
+  // pass (register arithmetic for Float64 data unless native FP64 was requested)
   if ((ps.op == OP_C2C || ps.op == OP_R2C || ps.op == OP_C2R) && M >= 2 && M <= 2048 &&
       !(P->rb == 8 && P->precision == PFGB_PRECISION_NATIVE)) {
     keep_generic();
@@ -1972,10 +1972,10 @@ static bool r2r_register_form(const pfgb_plan* P, int kind, int64_t n) {
 // gathered into packed complex lines (two real lines per complex line for
 // real data: every kind has a real kernel), the m-point c2c transform, and
 // the outputs read from it.  Taken where the extension is beyond the generic
-// kernel's core (split or Bluestein c2c), and in Float64 plans for every line
-// without a register form of its own whose extension is a one-pass length:
-// the c2c pass then runs in double-float on a register kernel instead of the
-// generic kernel's native FP64.
+// kernel's core (split or Bluestein c2c), and in Float64 plans for lines of a
+// one-pass extension that neither a power-of-two form nor the smooth-length pass
+// takes (a prime factor above 7 in the DFT's length): the c2c pass then runs on a
+// register kernel instead of the generic kernel's native FP64.
 static bool expand_long_r2r(const pfgb_plan* P, const Pass& ps, Pass& pre, Pass& c, Pass& post) {
   if (ps.pk != PK_TRANSFORM || (ps.op != OP_R2R_C && ps.op != OP_R2R_R)) return false;
   const int a = ps.axis;

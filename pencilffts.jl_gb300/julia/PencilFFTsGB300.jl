@@ -79,8 +79,8 @@ struct PlanInfo
     n_passes_backward::Int32
 end
 
-# PFGB_PRECISION_* (include/pencilfft_gb300.h): :default (Float64 power-of-two
-# lines in double-float), :native (FP64 everywhere), :tc (Float32 tensor-core
+# PFGB_PRECISION_* (include/pencilfft_gb300.h): :default (Float64 lines on the
+# integer and FP32 pipes), :native (FP64 everywhere), :tc (Float32 tensor-core
 # split form), :fx (Float64 block floating point)
 const PRECISION = Dict(:default => Int32(0), :native => Int32(1), :tc => Int32(2), :fx => Int32(3))
 
